@@ -8,12 +8,13 @@
 //   k_mux             k_ft_array_mux (1014)
 //   k_gather/k_scatter/k_scatter_zero/k_gather_range/k_scatter_range
 //                     k_ft_array_{get_subset,assign_to_subset,assign_zero_to_subset,get_range,assign_to_range} (390-515)
-//   k_encode          k_ft_array_to_bytes_folded (629), batched inversion
+//   k_zinv            k_ft_array_to_bytes_folded (629) / k_ft_array_to_bytes_affine (659), batched inversion
 //   k_decode          k_ft_array_from_bytes_folded (735)
-//   k_to_affine       k_ft_array_to_bytes_affine (659)  k_from_affine k_ft_array_from_bytes_affine (793)
+//   k_from_affine     k_ft_array_from_bytes_affine (793)
 //   k_validate        k_ft_array_validate (859)
 #include "internal.h"
 #include "points.cuh"
+#include "fe_inv.cuh"
 
 #define FT_TABLE_QUAL static __constant__
 #define FT_WANT_L_SLIDE
@@ -197,93 +198,88 @@ __global__ void __launch_bounds__(256) k_scatter_range(uint4 *d, size_t ds, cons
 
 // ------------------------------------------------------------ wire formats
 
-// Batched inversion (Montgomery's trick) over K consecutive points per
-// thread: one fe_invert and 3(K-1) multiplications instead of K inversions.
-// A zero Z is replaced by 1 inside the product and its inverse reported as 0,
-// which is what fe25519_invert(0) = 0 gives the reference.
-template <int K, class Emit>
-FT_DEV void batch_zinv(const uint4 *p, size_t s, size_t n, size_t base, Emit emit)
+// Canonical outputs that divide by Z (folded and affine encodings): K points
+// per thread share one division-step inversion (fe_inv) by Montgomery's
+// trick, 3 multiplications per point more.  A zero Z counts as 1 inside the
+// product and its inverse as 0, which is what fe25519_invert(0) = 0 gives
+// the reference.  Thread t of a warp takes the points 32 k + t of the warp's
+// 32 K, so its loads and stores are those of whole warps; the products of
+// the earlier points wait in shared memory (32 bytes per point).
+static constexpr int ZINV_NT = 128;
+
+FT_DEV void load_z(fe &z, uint32_t &zero_mask, const uint4 *p, size_t s, size_t n, size_t i)
 {
-    fe q[K];
-    uint32_t zero_bits = 0;
-    fe acc;
-    fe_1(acc);
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-        size_t i = base + k;
-        fe z;
-        if (i < n) fe_from_u4(z, p[4 * s + i], p[5 * s + i]);
-        else fe_1(z);
-        uint32_t zm = 0u - (uint32_t)fe_iszero(z);
-        zero_bits |= (zm & 1u) << k;
-        fe one;
-        fe_1(one);
-        fe_cmov(z, one, zm);
-        if (k == 0) fe_copy(acc, z);
-        else fe_mul(acc, acc, z);
-        fe_copy(q[k], acc);
+    if (i < n) fe_from_u4(z, p[4 * s + i], p[5 * s + i]);
+    else fe_1(z);
+    zero_mask = 0u - (uint32_t)fe_iszero(z);
+    fe one;
+    fe_1(one);
+    fe_cmov(z, one, zero_mask);
+}
+
+struct EmitFolded {
+    static constexpr int WORDS = 2; // uint4 words per point
+    FT_DEV static void emit(uint4 *o, const fe &x, const fe &y)
+    {
+        fe yc;
+        fe_canon(yc, y);
+        yc.v[7] ^= fe_isnegative(x) << 31;
+        o[0] = u4_lo(yc);
+        o[1] = u4_hi(yc);
+    }
+};
+
+struct EmitAffine {
+    static constexpr int WORDS = 4;
+    FT_DEV static void emit(uint4 *o, const fe &x, const fe &y)
+    {
+        fe xc, yc;
+        fe_canon(xc, x);
+        fe_canon(yc, y);
+        o[0] = u4_lo(xc);
+        o[1] = u4_hi(xc);
+        o[2] = u4_lo(yc);
+        o[3] = u4_hi(yc);
+    }
+};
+
+template <class Emit>
+__global__ void __launch_bounds__(ZINV_NT) k_zinv(uint4 *out, const uint4 *p, size_t s, size_t n, int K)
+{
+    extern __shared__ uint4 pre[]; // [k][2][ZINV_NT]: product of the thread's first k points
+    uint4 *my = pre + threadIdx.x;
+    const size_t base = ((size_t)blockIdx.x * (ZINV_NT / 32) + (threadIdx.x >> 5)) * 32 * K + (threadIdx.x & 31);
+    fe acc, z;
+    uint32_t zm;
+    load_z(acc, zm, p, s, n, base);
+#pragma unroll 1
+    for (int k = 1; k < K; ++k) {
+        my[(2 * k) * ZINV_NT] = u4_lo(acc);
+        my[(2 * k + 1) * ZINV_NT] = u4_hi(acc);
+        load_z(z, zm, p, s, n, base + 32 * (size_t)k);
+        fe_mul(acc, acc, z);
     }
     fe inv;
-    fe_invert(inv, acc);
-#pragma unroll
+    fe_inv(inv, acc);
+#pragma unroll 1
     for (int k = K - 1; k >= 0; --k) {
-        size_t i = base + k;
-        fe zinv;
-        if (k > 0) {
-            fe_mul(zinv, inv, q[k - 1]);
-            fe z;
-            if (i < n) fe_from_u4(z, p[4 * s + i], p[5 * s + i]);
-            else fe_1(z);
-            fe one;
-            fe_1(one);
-            fe_cmov(z, one, 0u - ((zero_bits >> k) & 1u));
-            fe_mul(inv, inv, z);
-        } else {
-            fe_copy(zinv, inv);
+        const size_t i = base + 32 * (size_t)k;
+        load_z(z, zm, p, s, n, i);
+        fe zinv = inv;
+        if (k) {
+            fe q;
+            fe_from_u4(q, my[(2 * k) * ZINV_NT], my[(2 * k + 1) * ZINV_NT]);
+            fe_mul_x2(zinv, inv, q, inv, inv, z);
         }
-        fe zero;
+        fe zero, x, y;
         fe_0(zero);
-        fe_cmov(zinv, zero, 0u - ((zero_bits >> k) & 1u));
-        if (i < n) emit(i, zinv);
-    }
-}
-
-template <int K>
-__global__ void __launch_bounds__(128) k_encode(uint4 *out, const uint4 *p, size_t s, size_t n)
-{
-    size_t groups = (n + K - 1) / K;
-    FT_GRID_LOOP(g, groups)
-    {
-        batch_zinv<K>(p, s, n, g * K, [&](size_t i, const fe &zinv) {
-            ge_p3 h;
-            ld_p3(h, p, s, i);
-            uint32_t w[8];
-            ge_encode_with_zinv(w, h, zinv);
-            out[2 * i] = make_uint4(w[0], w[1], w[2], w[3]);
-            out[2 * i + 1] = make_uint4(w[4], w[5], w[6], w[7]);
-        });
-    }
-}
-
-template <int K>
-__global__ void __launch_bounds__(128) k_to_affine(uint4 *out, const uint4 *p, size_t s, size_t n)
-{
-    size_t groups = (n + K - 1) / K;
-    FT_GRID_LOOP(g, groups)
-    {
-        batch_zinv<K>(p, s, n, g * K, [&](size_t i, const fe &zinv) {
-            ge_p3 h;
-            ld_p3(h, p, s, i);
-            fe x, y;
-            fe_mul(x, h.X, zinv);
-            fe_mul(y, h.Y, zinv);
-            fe_canon(x, x);
-            fe_canon(y, y);
-            out[4 * i + 0] = u4_lo(x);
-            out[4 * i + 1] = u4_hi(x);
-            out[4 * i + 2] = u4_lo(y);
-            out[4 * i + 3] = u4_hi(y);
-        });
+        fe_cmov(zinv, zero, zm);
+        if (i < n) {
+            fe_from_u4(x, p[0 * s + i], p[1 * s + i]);
+            fe_from_u4(y, p[2 * s + i], p[3 * s + i]);
+            fe_mul_x2(x, x, zinv, y, y, zinv);
+            Emit::emit(out + Emit::WORDS * i, x, y);
+        }
     }
 }
 
@@ -582,17 +578,41 @@ cudaError_t to_packed(uint8_t *o, View v, size_t n, cudaStream_t st) { FT_LAUNCH
 cudaError_t from_packed(View v, const uint8_t *in, size_t n, cudaStream_t st) { FT_LAUNCH(k_from_packed, n, 256, v.p, v.s, (const uint4 *)in, n); }
 cudaError_t validate(View v, size_t n, long long *bad, cudaStream_t st) { FT_LAUNCH(k_validate, n, 128, v.p, v.s, n, bad); }
 
-static const int ENC_K = 8;
-cudaError_t encode(uint8_t *o, View v, size_t n, cudaStream_t st)
+// Points per inversion: an inversion costs a warp scheduler 30,000 to 39,000
+// cycles (19 us alone) and a point in the loops about 5,000 (2 us), so the
+// points go one to a thread until every scheduler has a warp (sm_count x 128
+// threads), and then into longer threads: one block per SM up to 18 points
+// a thread, two, three (72 KB of shared memory each), each launch one wave.
+// Measured (n: this K, one point a thread, the earlier 8 points per chain of
+// 254 squarings): 16: 25, 25, 90 us; 65,536: 31 (K = 4), 71, 87 us;
+// 200,003: 47 (12), 177, 88 us; 1,048,576: 158 (12), 838, 314 us.
+static constexpr int ZINV_MAX_K = 18;
+static int zinv_points(size_t n)
 {
-    size_t groups = (n + ENC_K - 1) / ENC_K;
-    FT_LAUNCH(k_encode<ENC_K>, groups, 128, (uint4 *)o, v.p, v.s, n);
+    const size_t per_sm = (size_t)sm_count() * ZINV_NT;
+    for (size_t blocks = 1; blocks <= 3; ++blocks) {
+        const size_t k = (n + blocks * per_sm - 1) / (blocks * per_sm);
+        if (k <= ZINV_MAX_K) return (int)k;
+    }
+    return ZINV_MAX_K;
 }
-cudaError_t to_affine(uint8_t *o, View v, size_t n, cudaStream_t st)
+
+template <class Emit>
+static cudaError_t zinv_launch(uint8_t *o, View v, size_t n, cudaStream_t st)
 {
-    size_t groups = (n + ENC_K - 1) / ENC_K;
-    FT_LAUNCH(k_to_affine<ENC_K>, groups, 128, (uint4 *)o, v.p, v.s, n);
+    if (n == 0) return cudaSuccess;
+    const int K = zinv_points(n);
+    const size_t smem = (size_t)K * 2 * ZINV_NT * sizeof(uint4);
+    const unsigned grid = (unsigned)((n + (size_t)ZINV_NT * K - 1) / ((size_t)ZINV_NT * K));
+    static SmemAttr attr;
+    cudaError_t e = ensure_smem_attr(attr, (const void *)k_zinv<Emit>, (size_t)ZINV_MAX_K * 2 * ZINV_NT * sizeof(uint4));
+    if (e != cudaSuccess) return e;
+    k_zinv<Emit><<<grid, ZINV_NT, smem, st>>>((uint4 *)o, v.p, v.s, n, K);
+    return cudaGetLastError();
 }
+
+cudaError_t encode(uint8_t *o, View v, size_t n, cudaStream_t st) { return zinv_launch<EmitFolded>(o, v, n, st); }
+cudaError_t to_affine(uint8_t *o, View v, size_t n, cudaStream_t st) { return zinv_launch<EmitAffine>(o, v, n, st); }
 
 cudaError_t copy_points(View d, View s, size_t n, cudaStream_t st)
 {
