@@ -11,7 +11,7 @@ namespace ft {
 
 // Latency-bound lengths: four lanes per point (quad.cuh), so that a window's
 // 36 multiplications and squarings take 10 in sequence instead of 36 (one
-// point: 345 us against 553 with one thread in the 128-thread kernel).  A
+// point: 244 us against 553 with one thread in the 128-thread kernel).  A
 // block of 128 threads holds 32 points; a thread keeps its coordinate of the
 // 8-entry table in shared memory, [entry][half][thread], and scans all of it
 // under masks for each digit, as the one-thread ladder does.
@@ -19,7 +19,9 @@ static constexpr int QUAD_NT = 128;
 
 __global__ void __launch_bounds__(QUAD_NT, 5) k_smul_quad(uint4 *p, size_t s, size_t n, const uint4 *sc, int sc_step)
 {
-    __shared__ uint4 smem[8 * 2 * QUAD_NT];
+    __shared__ uint4 smem[8 * 2 * QUAD_NT], trade[4 * QUAD_NT];
+    QuadX x(trade, QUAD_NT);
+    const uint32_t m013 = quad_mask(threadIdx.x & 3, 11);
     uint4 *tab = smem + threadIdx.x;
     const int l = threadIdx.x & 3;
     const size_t i = ((size_t)blockIdx.x * QUAD_NT + threadIdx.x) >> 2;
@@ -38,7 +40,7 @@ __global__ void __launch_bounds__(QUAD_NT, 5) k_smul_quad(uint4 *p, size_t s, si
     // (P + 4P, P + 2P), 6P (a doubling), 7P (P + 6P): the reference's
     // formula for each, with P and the last point live
     v = P;
-    quad_cached(c, v, l);
+    quad_cached(c, v, x);
     tab[0] = u4_lo(c);
     tab[QUAD_NT] = u4_hi(c);
 #pragma unroll 1
@@ -47,12 +49,12 @@ __global__ void __launch_bounds__(QUAD_NT, 5) k_smul_quad(uint4 *p, size_t s, si
             const int e = 0x5013000 >> (4 * step) & 7;
             fe_from_u4(c, tab[2 * e * QUAD_NT], tab[(2 * e + 1) * QUAD_NT]);
             v = P;
-            quad_add(v, c, l);
+            quad_add(v, c, x);
         } else {
-            quad_dbl(v, l);
+            quad_dbl(v, x);
         }
-        quad_p3(v, l);
-        quad_cached(c, v, l);
+        quad_p3(v, x);
+        quad_cached(c, v, x);
         const int e = 0x6524731 >> (4 * step) & 7;
         tab[2 * e * QUAD_NT] = u4_lo(c);
         tab[(2 * e + 1) * QUAD_NT] = u4_hi(c);
@@ -75,17 +77,18 @@ __global__ void __launch_bounds__(QUAD_NT, 5) k_smul_quad(uint4 *p, size_t s, si
         }
         // -P: Y+X and Y-X trade lanes, T2d is negated
         fe o;
-        quad_shfl(o, c, l ^ 2);
+        x.put(c);
+        x.get(o, l ^ 2);
         fe_neg(t, c);
-        fe_select(t, l == 0, t, o);
-        fe_cmov(c, t, l == 2 ? 0u : nm);
-        quad_add(v, c, l);
-        quad_p3(v, l);
+        fe_pick(t, o, t, x.m0);
+        fe_cmov(c, t, nm & m013);
+        quad_add(v, c, x);
+        quad_p3(v, x);
         if (w == 0) break;
 #pragma unroll 1
         for (int k = 0; k < 4; ++k) {
-            quad_dbl(v, l);
-            quad_p3(v, l);
+            quad_dbl(v, x);
+            quad_p3(v, x);
         }
         d = pop_top_nibble(b) - 8;
     }
@@ -125,19 +128,20 @@ static cudaError_t smul_quad(View v, size_t n, const uint4 *sc, int sc_step, cud
 // Fewer points than a wave of the 384-thread ladder (384 per SM) cost a whole
 // one: twelve warps on each SM share its pipe for 1,134 us, on one SM or on
 // all.  Measured with 152 SMs, us per launch by points per SM:
-//               <= 32   <= 64   <= 96  <= 128  <= 192  <= 224  <= 256  <= 384
-//   quad           345     436     504     634     951       -    1179    1720
-//   128 threads    553     553     553     553    1106    1106    1106    1657
+//               <= 32   <= 64   <= 96  <= 128  <= 160  <= 224  <= 256  <= 384
+//   quad           244     317     441     567     688     941    1070    1569
+//   128 threads    553     553     553     554    1106    1106    1106    1657
 //   224 threads    771     775     775     776     776     776    1538    1544
 //   384 threads   1130    1133    1133    1134    1134    1134    1134    1135
-// so the points go to four lanes each up to 96 per SM, then to one warp per
-// scheduler, then to the largest block with its tables in shared memory.
+// so the points go to four lanes each up to 160 per SM, then to the largest
+// block with its tables in shared memory, and to four lanes again between the
+// points that holds and 256 per SM.
 static cudaError_t smul_part_wave(View v, size_t n, const uint4 *sc, int sc_step, cudaStream_t st)
 {
     const size_t sm = (size_t)sm_count();
-    if (n <= 96 * sm) return smul_quad(v, n, sc, sc_step, st);
-    if (n <= 128 * sm) return ladder_launch_128(v.p, v.s, n, sc, sc_step, st);
+    if (n <= 160 * sm) return smul_quad(v, n, sc, sc_step, st);
     if (n <= 224 * sm) return ladder_launch_224(v.p, v.s, n, sc, sc_step, st);
+    if (n <= 256 * sm) return smul_quad(v, n, sc, sc_step, st);
     return ladder_launch_384(v.p, v.s, n, sc, sc_step, st);
 }
 
@@ -158,7 +162,7 @@ cudaError_t smul_var(View v, size_t n, const uint8_t *sc, int sc_step, cudaStrea
     }
     const size_t sm = (size_t)sm_count(), wave = 384 * sm, rest = n % wave;
     if (n < wave) return smul_part_wave(v, n, s4, sc_step, st);
-    const size_t bulk = rest > 224 * sm ? n : n - rest;
+    const size_t bulk = rest > 256 * sm ? n : n - rest;
     cudaError_t e = ladder_launch_384(v.p, v.s, bulk, s4, sc_step, st);
     if (e != cudaSuccess || bulk == n) return e;
     return smul_part_wave(View{v.p + bulk, v.s}, rest, s4 + 2 * bulk * (size_t)sc_step, sc_step, st);

@@ -13,24 +13,59 @@
 // so that p1p1 to p3 is one product with the next lane's value: E H = T,
 // H G = Y, G F = Z, F E = X.  The operands and the order of every field
 // operation are those of ge.cuh, so coordinates are the same words.  All
-// lanes of a warp run these together (full-mask shuffles).
+// lanes of a warp run these together.
 #pragma once
 #include "ge.cuh"
 #include "u4.cuh"
 
 namespace ft {
 
-FT_DEV void quad_shfl(fe &o, const fe &v, int src)
+// b where the mask is set, else a
+FT_DEV void fe_pick(fe &h, const fe &a, const fe &b, uint32_t m)
 {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) o.v[k] = __shfl_sync(0xffffffffu, v.v[k], src, 4);
+    for (int k = 0; k < 8; ++k) h.v[k] = (a.v[k] & ~m) | (b.v[k] & m);
 }
 
-FT_DEV void fe_select(fe &h, bool c, const fe &a, const fe &b)
+// all ones in the lanes l of `lanes`; opaque, so that a pick stays a pick (as a
+// condition the compiler branches around each one's eight moves: a point's
+// ladder 345 us against 244)
+FT_DEV uint32_t quad_mask(int l, unsigned lanes)
 {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) h.v[k] = c ? a.v[k] : b.v[k];
+    uint32_t m = 0u - (lanes >> l & 1u);
+    asm volatile("" : "+r"(m));
+    return m;
 }
+
+// Lanes trade values through shared memory, two uint4 a thread in one of two
+// buffers in turn (`slot`): a value written once is read by any number of
+// lanes, and one warp barrier orders it (a shuffle moves one word and brings a
+// barrier of its own).
+struct QuadX {
+    uint4 *slot; // this thread's, buffer 0: [buffer][half][thread], 4 * threads uint4
+    int stride;  // threads of the block
+    int l;       // the lane's place in its quad
+    uint32_t m0, m1, m03, m13, m23; // quad_mask of those lanes
+    int flip = 0;
+    FT_DEV QuadX(uint4 *buf, int threads)
+        : slot(buf + threadIdx.x), stride(threads), l(threadIdx.x & 3), m0(quad_mask(l, 1)), m1(quad_mask(l, 2)),
+          m03(quad_mask(l, 9)), m13(quad_mask(l, 10)), m23(quad_mask(l, 12))
+    {
+    }
+    FT_DEV void put(const fe &v)
+    {
+        flip ^= 2 * stride;
+        slot[flip] = u4_lo(v);
+        slot[flip + stride] = u4_hi(v);
+        __syncwarp();
+    }
+    // the value that lane `src` of the quad put last
+    FT_DEV void get(fe &o, int src) const
+    {
+        const uint4 *q = slot + flip + src - l;
+        fe_from_u4(o, q[0], q[stride]);
+    }
+};
 
 // a + b for m = 0 (the words of fe_add), a - b for m = all ones (fe_sub's)
 FT_DEV void fe_addsub(fe &h, const fe &a, const fe &b, uint32_t m)
@@ -51,65 +86,68 @@ FT_DEV void fe_addsub(fe &h, const fe &a, const fe &b, uint32_t m)
 }
 
 // p1p1 to p3
-FT_DEV void quad_p3(fe &v, int l)
+FT_DEV void quad_p3(fe &v, QuadX &x)
 {
     fe o;
-    quad_shfl(o, v, (l + 1) & 3);
+    x.put(v);
+    x.get(o, (x.l + 1) & 3);
     fe_mul(v, v, o);
 }
 
 // p3 (T unused) doubled, to p1p1 (ge_p2_dbl)
-FT_DEV void quad_dbl(fe &v, int l)
+FT_DEV void quad_dbl(fe &v, QuadX &x)
 {
-    fe x, y, t, s;
-    quad_shfl(x, v, 3);
-    quad_shfl(y, v, 1);
-    fe_add(t, x, y);
-    fe_select(t, l == 0, t, v);
+    fe a, b, t, s;
+    x.put(v);
+    x.get(a, 3);
+    x.get(b, 1);
+    fe_add(t, a, b);
+    fe_pick(t, v, t, x.m0);
     fe_sq(s, t); // (X+Y)^2, Y^2, Z^2, X^2
-    quad_shfl(y, s, 1);
-    quad_shfl(x, s, 3);
-    fe_add(t, s, s);
-    quad_shfl(t, t, 2);                              // 2 Z^2
-    fe_addsub(v, y, x, l < 2 ? 0u : ~0u);            // lanes 0, 1: H; lanes 2, 3: G
-    fe_select(t, l == 0, s, t);
-    fe_sub(t, t, v);                                 // lane 0: E, lane 3: F
-    fe_select(v, l == 0 || l == 3, t, v);
+    x.put(s);
+    x.get(a, 1);
+    x.get(b, 3);
+    x.get(t, 2);
+    fe_add(t, t, t);           // 2 Z^2
+    fe_addsub(v, a, b, x.m23); // lanes 0, 1: H; lanes 2, 3: G
+    fe_pick(t, t, s, x.m0);
+    fe_sub(t, t, v);           // lane 0: E, lane 3: F
+    fe_pick(v, v, t, x.m03);
 }
 
-// the point's Y in y and X in x, in lanes 1 and 3
-FT_DEV void quad_yx(fe &y, fe &x, const fe &v, int l)
+// Y + X in lane 1, Y - X in lane 3, v in the others
+FT_DEV void quad_yx(fe &t, const fe &v, QuadX &x)
 {
-    fe o;
-    quad_shfl(o, v, l ^ 2);
-    fe_select(y, l == 1, v, o);
-    fe_select(x, l == 1, o, v);
+    fe o, a, b;
+    x.put(v);
+    x.get(o, x.l ^ 2);
+    fe_pick(b, o, v, x.m1);
+    fe_pick(a, v, o, x.m1);
+    fe_addsub(o, b, a, ~x.m1);
+    fe_pick(t, v, o, x.m13);
 }
 
 // p3 plus cached, to p1p1 (ge_add)
-FT_DEV void quad_add(fe &v, const fe &q, int l)
+FT_DEV void quad_add(fe &v, const fe &q, QuadX &x)
 {
-    fe y, x, t, s, d;
-    quad_yx(y, x, v, l);
-    fe_addsub(t, y, x, l == 3 ? ~0u : 0u);
-    fe_select(t, l & 1, t, v);
+    fe a, b, t, s;
+    quad_yx(t, v, x);
     fe_mul(s, t, q); // T T2d, (Y+X)(Y+X)', Z Z', (Y-X)(Y-X)'
-    fe_add(d, s, s);
-    fe_select(d, l == 2, d, s);
-    quad_shfl(y, d, l < 2 ? 1 : 2);
-    quad_shfl(x, s, l < 2 ? 3 : 0);
-    fe_addsub(v, y, x, l == 0 || l == 3 ? ~0u : 0u);
+    x.put(s);
+    x.get(b, x.l < 2 ? 1 : 2);
+    x.get(a, x.l < 2 ? 3 : 0);
+    fe_add(t, b, b);
+    fe_pick(b, b, t, x.m23);
+    fe_addsub(v, b, a, x.m03);
 }
 
 // p3 to cached (ge_p3_to_cached)
-FT_DEV void quad_cached(fe &c, const fe &v, int l)
+FT_DEV void quad_cached(fe &c, const fe &v, QuadX &x)
 {
-    fe y, x, t;
-    quad_yx(y, x, v, l);
-    fe_addsub(t, y, x, l == 3 ? ~0u : 0u);
+    fe t;
+    quad_yx(t, v, x);
     fe_mul(c, v, fe_d2());
-    fe_select(c, l == 0, c, v);
-    fe_select(c, l & 1, t, c);
+    fe_pick(c, t, c, x.m0);
 }
 
 // the lane's coordinate of point i (identity past n)

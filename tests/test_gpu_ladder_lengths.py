@@ -1,6 +1,6 @@
 """ft_mul and ft_scale at the lengths where the ladder's launch changes (with
-152 SMs): four lanes per point up to 96 points per SM, the 128- and 224-thread
-kernels, whole waves of 384 per SM with a rest in a second launch.  Exact:
+152 SMs): four lanes per point up to 160 points per SM, the 224-thread kernel, four
+lanes again up to 256, whole waves of 384 with a rest in a second launch.  Exact:
 the oracle's coordinates, word for word, edge scalars among them."""
 import numpy as np
 import pytest
@@ -25,8 +25,8 @@ def pool(orc):
     return pts, k, orc.mul(pts, k, threads=8), orc.mul(pts, np.repeat(k[:1], n, axis=0), threads=8)
 
 
-@pytest.mark.parametrize("n", [1, 7, 8, 9, 33, 32 * SM + 1, 96 * SM, 96 * SM + 1, 128 * SM + 1, 224 * SM + 1, 384 * SM,
-                               384 * SM + 1, (384 + 96) * SM + 5, (384 + 224) * SM + 1])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 33, 32 * SM + 1, 96 * SM + 1, 160 * SM, 160 * SM + 1, 224 * SM + 1, 256 * SM + 1,
+                               384 * SM, 384 * SM + 1, (384 + 160) * SM + 5, (384 + 256) * SM + 1])
 def test_lengths(ft, pool, n):
     pts, k, products, scaled = pool
     idx = np.arange(n) % len(pts)
