@@ -71,6 +71,8 @@ FT_DEV void shr5_288(uint32_t c[9])
 static constexpr int ENC_SEL_GROUP = FT_ENC_SEL_GROUP;
 static_assert(ENC_ENTRIES % ENC_SEL_GROUP == 0, "select grouping");
 
+// (S: the stride of the table's words in uint4.)
+template <int S = 1>
 FT_DEV void enc_select(ge_precomp &t, int d, const uint4 *row)
 {
     const uint32_t bneg = (uint32_t)d >> 31;
@@ -85,11 +87,11 @@ FT_DEV void enc_select(ge_precomp &t, int d, const uint4 *row)
     for (int k = 0; k < ENC_ENTRIES; k += ENC_SEL_GROUP) {
 #pragma unroll
         for (int q = 0; q < ENC_SEL_GROUP; ++q) {
-            const uint4 *e = row + 6 * (k + q);
+            const uint4 *e = row + 6 * S * (k + q);
             fe e0, e1, e2;
-            fe_from_u4(e0, e[0], e[1]);
-            fe_from_u4(e1, e[2], e[3]);
-            fe_from_u4(e2, e[4], e[5]);
+            fe_from_u4(e0, e[0 * S], e[1 * S]);
+            fe_from_u4(e1, e[2 * S], e[3 * S]);
+            fe_from_u4(e2, e[4 * S], e[5 * S]);
             const uint32_t m = ct_eq_mask(babs, (uint32_t)(k + q + 1));
 #pragma unroll
             for (int i = 0; i < 8; ++i) {

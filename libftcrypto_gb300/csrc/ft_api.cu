@@ -33,19 +33,24 @@ struct Ctx {
     size_t scratch_cap = 0;
     long long *d_status = nullptr; // one device word for "last bad index"
     ft_error last_void = FT_ERR_NO_ERROR;
-    // encryption tables (B's and a public key's) of the last PK_CACHE keys
-    // used, least recently used replaced: a table costs ~0.55 ms to build
-    // (255 doublings in sequence for its last row), so callers alternating
-    // between a few keys build each once
+    // comb tables of the last PK_CACHE public keys used, least recently used
+    // replaced: a key's base points are a chain of 255 doublings, so callers
+    // alternating between a few keys build each once; its radix-256 table
+    // waits for the first call long enough to read it
     struct KeyTab {
         uint8_t pk[32];
-        uint32_t *table = nullptr;
+        ft::CombTable t;
+        bool wide = false;
         uint64_t used = 0; // 0: empty
     };
     static constexpr int PK_CACHE = 4;
     KeyTab keys[PK_CACHE];
     uint64_t key_clock = 0;
-    uint32_t *b_table = nullptr;  // radix-32 comb table of B (fixed-base products)
+    ft::CombTable b; // B's tables (fixed-base products)
+    // set by a kernel whose bounded wait ran out (mapped host memory): its
+    // results are not valid, and every later call reports it
+    volatile int *fault = nullptr;
+    int *d_fault = nullptr;
     void *dlog_mem = nullptr;     // decryption table of j*B, j < dlog.m_max
     ft::DlogTable dlog;
     // Transfers that overlap queued kernels (see export_begin, stage_scalars):
@@ -91,6 +96,7 @@ ft_error map_err(cudaError_t e)
             ft_error _ie = ft_crypto_init();            \
             if (_ie) return _ie;                        \
         }                                               \
+        if (*g.fault) return FT_ERR_INTERNAL_LIBRARY_ERROR; \
     } while (0)
 
 cudaError_t dev_alloc(void **p, size_t bytes)
@@ -258,7 +264,7 @@ ft_error export_to_host(uint8_t *mem, const_ft_ge25519_array a, size_t bpp, Conv
         start = end;
     }
     CK(cudaStreamSynchronize(st));
-    return FT_ERR_NO_ERROR;
+    return *g.fault ? FT_ERR_INTERNAL_LIBRARY_ERROR : FT_ERR_NO_ERROR;
 }
 
 // Copies `bytes` of pinned host memory into one of two staging buffers on
@@ -398,9 +404,9 @@ ft_error status_read(int64_t *res)
     return FT_ERR_NO_ERROR;
 }
 
-// the encryption tables of B and of the public key pk (32-byte folded
-// encoding) into d_tables (ENC_TABLES_BYTES), queued on the library stream
-ft_error build_key_tables(uint32_t *d_tables, const uint8_t *pk)
+// the base points and the radix-32 table of the public key pk (32-byte folded
+// encoding) into t (COMB_TABLE_BYTES), queued on the library stream
+ft_error build_key_table(ft::CombTable t, const uint8_t *pk)
 {
     ft_ge25519_array q;
     int64_t bad = -1;
@@ -410,34 +416,40 @@ ft_error build_key_tables(uint32_t *d_tables, const uint8_t *pk)
         ft_array_free(q);
         return FT_ERR_INVALID_POINT;
     }
-    cudaError_t e = cudaMemcpyAsync(d_tables, g.b_table, ft::ENC_TABLE_WORDS * 4, cudaMemcpyDeviceToDevice, g.stream);
-    if (e == cudaSuccess) e = ft::build_enc_table(d_tables + ft::ENC_TABLE_WORDS, ft::view_of(q), g.stream);
+    cudaError_t e = ft::comb_bases(t, ft::view_of(q), g.stream);
+    if (e == cudaSuccess) e = ft::comb_t32(t, g.stream);
     ft_array_free(q);
     CK(e);
     return FT_ERR_NO_ERROR;
 }
 
-// the encryption tables of pk, from the cache or built into its least
-// recently used slot (kernels still queued on the library stream that read
-// the slot's old tables run before the rebuild, in stream order)
-ft_error ensure_pk_table(const uint8_t *pk, const uint32_t **tables)
+// the tables of pk for a call over n ciphertexts, from the cache or built
+// into its least recently used slot (kernels still queued on the library
+// stream that read the slot's old tables run before the rebuild, in stream
+// order)
+ft_error ensure_pk_table(const uint8_t *pk, size_t n, const ft::CombTable **table)
 {
     Ctx::KeyTab *slot = &g.keys[0];
+    bool found = false;
     for (Ctx::KeyTab &k : g.keys) {
-        if (k.used && std::memcmp(k.pk, pk, 32) == 0) {
-            k.used = ++g.key_clock;
-            *tables = k.table;
-            return FT_ERR_NO_ERROR;
-        }
-        if (k.used < slot->used) slot = &k;
+        found = k.used && std::memcmp(k.pk, pk, 32) == 0;
+        if (found || k.used < slot->used) slot = &k;
+        if (found) break;
     }
-    slot->used = 0;
-    if (!slot->table) CK(dev_alloc((void **)&slot->table, ft::ENC_TABLES_BYTES));
-    ft_error err = build_key_tables(slot->table, pk);
-    if (err) return err;
-    std::memcpy(slot->pk, pk, 32);
+    if (!found) {
+        slot->used = 0;
+        slot->wide = false;
+        if (!slot->t.mem) CK(dev_alloc((void **)&slot->t.mem, ft::COMB_TABLE_BYTES));
+        ft_error err = build_key_table(slot->t, pk);
+        if (err) return err;
+        std::memcpy(slot->pk, pk, 32);
+    }
     slot->used = ++g.key_clock;
-    *tables = slot->table;
+    if (!slot->wide && ft::comb_is_wide(2 * n)) {
+        CK(ft::comb_t256(slot->t, g.stream));
+        slot->wide = true;
+    }
+    *table = &slot->t;
     return FT_ERR_NO_ERROR;
 }
 
@@ -460,7 +472,7 @@ ft_error ensure_dlog(uint64_t m_max)
     uint64_t *js = (uint64_t *)((uint8_t *)s + b_pts);
     uint8_t *enc = (uint8_t *)s + b_pts + b_js;
     if (e == cudaSuccess) e = ft::iota_u64(js, m_max, g.stream);
-    if (e == cudaSuccess) e = ft::smul_base_small(pts, m_max, js, g.b_table, g.stream);
+    if (e == cudaSuccess) e = ft::smul_base_small(pts, m_max, js, g.b, g.d_fault, g.stream);
     if (e == cudaSuccess) e = ft::encode(enc, pts, m_max, g.stream);
     if (e == cudaSuccess) e = ft::dlog_build(g.dlog, mem, m_max, cap, enc, g.stream);
     if (e != cudaSuccess) {
@@ -499,7 +511,7 @@ const char *ft_error_str(ft_error err)
 
 namespace {
 
-// the library's stream, memory pool, status word and B's comb table
+// the library's stream, memory pool, status words and B's comb tables
 ft_error init_device(int dev)
 {
     CK(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
@@ -518,18 +530,25 @@ ft_error init_device(int dev)
     CK(cudaMemPoolSetAttribute(g.pool, cudaMemPoolAttrReleaseThreshold, &thr));
     g.device = dev;
     CK(cudaMallocFromPoolAsync((void **)&g.d_status, 256, g.pool, g.stream));
-    // the comb table of B, from B's encoding (y = 4/5, x even)
+    void *fault = nullptr;
+    CK(cudaHostAlloc(&fault, sizeof(int), cudaHostAllocMapped));
+    g.fault = (volatile int *)fault;
+    *g.fault = 0;
+    CK(cudaHostGetDevicePointer((void **)&g.d_fault, fault, 0));
+    // the comb tables of B, from B's encoding (y = 4/5, x even)
     uint8_t benc[32];
     std::memset(benc, 0x66, 32);
     benc[0] = 0x58;
     void *s;
-    CK(dev_alloc((void **)&g.b_table, ft::ENC_TABLE_WORDS * 4));
+    CK(dev_alloc((void **)&g.b.mem, ft::COMB_TABLE_BYTES));
     CK(dev_alloc(&s, align256(FT_PLANES_BYTES_PER_POINT) + 256));
     ft::View bp{(uint4 *)s, 1};
     uint8_t *d_enc = (uint8_t *)s + align256(FT_PLANES_BYTES_PER_POINT);
     CK(cudaMemcpyAsync(d_enc, benc, 32, cudaMemcpyHostToDevice, g.stream));
     CK(ft::decode(bp, d_enc, 1, g.d_status, g.stream));
-    CK(ft::build_enc_table(g.b_table, bp, g.stream));
+    CK(ft::comb_bases(g.b, bp, g.stream));
+    CK(ft::comb_t32(g.b, g.stream));
+    CK(ft::comb_t256(g.b, g.stream));
     CK(cudaStreamSynchronize(g.stream)); // benc is on the stack
     dev_free(s);
     CK(cudaStreamSynchronize(g.stream));
@@ -547,6 +566,7 @@ void init_release()
     }
     for (auto &ev : g.in_ev)
         if (ev) cudaEventDestroy(ev);
+    if (g.fault) cudaFreeHost((void *)g.fault);
     if (g.pool) cudaMemPoolDestroy(g.pool); // releases its memory once nothing is outstanding
     if (g.xfer) cudaStreamDestroy(g.xfer);
     if (g.stream) cudaStreamDestroy(g.stream);
@@ -602,7 +622,7 @@ ft_error ft_array_init_scalar(ft_ge25519_array *array, size_t n, const uint8_t *
         void *s;
         CK(scratch(&s, 256));
         CK(h2d(s, scalar, 32));
-        CK(ft::smul_base(ft::view_of(a), 1, (const uint8_t *)s, 0, g.b_table, g.stream));
+        CK(ft::smul_base(ft::view_of(a), 1, (const uint8_t *)s, 0, g.b, g.d_fault, g.stream));
         CK(ft::broadcast(ft::view_of(a, 1), n - 1, ft::view_of(a), g.stream));
         return FT_ERR_NO_ERROR;
     });
@@ -818,7 +838,7 @@ ft_error ft_array_from_scalars(ft_ge25519_array *array, const uint8_t *scalars, 
         void *s;
         CK(scratch(&s, align256(n * 32)));
         CK(h2d(s, scalars, n * 32));
-        CK(ft::smul_base(ft::view_of(a), n, (const uint8_t *)s, 1, g.b_table, g.stream));
+        CK(ft::smul_base(ft::view_of(a), n, (const uint8_t *)s, 1, g.b, g.d_fault, g.stream));
         return FT_ERR_NO_ERROR;
     });
 }
@@ -831,7 +851,7 @@ ft_error ft_array_from_small_scalars(ft_ge25519_array *array, const uint64_t *sm
         void *s;
         CK(scratch(&s, align256(n * 8)));
         CK(h2d(s, small, n * 8));
-        CK(ft::smul_base_small(ft::view_of(a), n, (const uint64_t *)s, g.b_table, g.stream));
+        CK(ft::smul_base_small(ft::view_of(a), n, (const uint64_t *)s, g.b, g.d_fault, g.stream));
         return FT_ERR_NO_ERROR;
     });
 }
@@ -1173,18 +1193,16 @@ ft_error ftx_mul_device(ft_ge25519_array array, const uint8_t *d_scalars, size_t
     return FT_ERR_NO_ERROR;
 }
 
-static int m_digits(unsigned bits) { return enc_digits(bits); }
-
 ft_error ftx_encrypt_device(ft_ge25519_array c1, ft_ge25519_array c2, const uint8_t *pk, const uint64_t *d_m,
                             const uint8_t *d_r, size_t n, unsigned bits)
 {
     ENSURE_INIT();
     if (bits < 1 || bits > 64) return FT_ERR_BAD_SIZE;
     if (c1->n != n || c2->n != n) return FT_ERR_SIZE_MISMATCH;
-    const uint32_t *tab;
-    ft_error err = ensure_pk_table(pk, &tab);
+    const ft::CombTable *tab;
+    ft_error err = ensure_pk_table(pk, n, &tab);
     if (err) return err;
-    CK(ft::encrypt(ft::view_of(c1), ft::view_of(c2), n, d_r, d_m, m_digits(bits), tab, g.stream));
+    CK(ft::encrypt(ft::view_of(c1), ft::view_of(c2), n, d_r, d_m, bits, g.b, *tab, g.d_fault, g.stream));
     CK(mark_ready(c1));
     CK(mark_ready(c2));
     return FT_ERR_NO_ERROR;
@@ -1199,7 +1217,7 @@ ft_error ftx_encrypt_device(ft_ge25519_array c1, ft_ge25519_array c2, const uint
 // the two launches take as many passes as one.  FT_ERR_BAD_SIZE if some
 // m_i >= 2^bits (the arrays' contents are then undefined).
 static ft_error encrypt_from_host(ft_ge25519_array a, ft_ge25519_array b, const uint64_t *m, const uint8_t *r,
-                                  size_t n, unsigned bits, const uint32_t *tab)
+                                  size_t n, unsigned bits, const ft::CombTable &tab)
 {
     if (n == 0) return FT_ERR_NO_ERROR;
     void *s;
@@ -1208,7 +1226,6 @@ static ft_error encrypt_from_host(ft_ge25519_array a, ft_ge25519_array b, const 
     uint8_t *dr = (uint8_t *)s;
     uint64_t *dm = (uint64_t *)(dr + br), *dacc = (uint64_t *)(dr + br + bm);
     const size_t first = std::min(n, ft::encrypt_pass());
-    const int mdig = m_digits(bits);
     CK(cudaMemcpyAsync(dr, r, first * 32, cudaMemcpyHostToDevice, g.stream));
     CK(cudaMemcpyAsync(dm, m, first * 8, cudaMemcpyHostToDevice, g.stream));
     CK(cudaEventRecord(g.in_ev[0], g.stream)); // the first part is copied (and the scratch free)
@@ -1218,11 +1235,11 @@ static ft_error encrypt_from_host(ft_ge25519_array a, ft_ge25519_array b, const 
         CK(cudaMemcpyAsync(dm + first, m + first, (n - first) * 8, cudaMemcpyHostToDevice, g.xfer));
         CK(cudaEventRecord(g.in_ev[1], g.xfer));
     }
-    CK(ft::encrypt(ft::view_of(a), ft::view_of(b), first, dr, dm, mdig, tab, g.stream));
+    CK(ft::encrypt(ft::view_of(a), ft::view_of(b), first, dr, dm, bits, g.b, tab, g.d_fault, g.stream));
     if (n > first) {
         CK(cudaStreamWaitEvent(g.stream, g.in_ev[1], 0));
-        CK(ft::encrypt(ft::view_of(a, first), ft::view_of(b, first), n - first, dr + first * 32, dm + first, mdig,
-                       tab, g.stream));
+        CK(ft::encrypt(ft::view_of(a, first), ft::view_of(b, first), n - first, dr + first * 32, dm + first, bits,
+                       g.b, tab, g.d_fault, g.stream));
     }
     CK(mark_ready(a));
     CK(mark_ready(b));
@@ -1243,8 +1260,8 @@ ft_error ftx_encrypt(ft_ge25519_array *c1, ft_ge25519_array *c2, const uint8_t *
     if (bits < 1 || bits > 64) return FT_ERR_BAD_SIZE;
     if (too_long(n)) return FT_ERR_OUT_OF_MEMORY;
     // the key's tables first (building them uses the scratch buffer)
-    const uint32_t *tab;
-    ft_error err = ensure_pk_table(pk, &tab);
+    const ft::CombTable *tab;
+    ft_error err = ensure_pk_table(pk, n, &tab);
     if (err) return err;
     ft_ge25519_array a, b;
     if ((err = arr_new(&a, n))) return err;
@@ -1252,7 +1269,7 @@ ft_error ftx_encrypt(ft_ge25519_array *c1, ft_ge25519_array *c2, const uint8_t *
         ft_array_free(a);
         return err;
     }
-    const ft_error res = encrypt_from_host(a, b, m, r, n, bits, tab);
+    const ft_error res = encrypt_from_host(a, b, m, r, n, bits, *tab);
     if (res) {
         ft_array_free(a); // stream-ordered: after any launch that writes it
         ft_array_free(b);
@@ -1295,10 +1312,10 @@ ft_error ftx_rerandomise_device(ft_ge25519_array c1, ft_ge25519_array c2, const 
 {
     ENSURE_INIT();
     if (c1->n != n || c2->n != n) return FT_ERR_SIZE_MISMATCH;
-    const uint32_t *tab;
-    ft_error err = ensure_pk_table(pk, &tab);
+    const ft::CombTable *tab;
+    ft_error err = ensure_pk_table(pk, n, &tab);
     if (err) return err;
-    CK(ft::rerandomise(ft::view_of(c1), ft::view_of(c2), n, d_r, tab, g.stream));
+    CK(ft::rerandomise(ft::view_of(c1), ft::view_of(c2), n, d_r, g.b, *tab, g.d_fault, g.stream));
     return FT_ERR_NO_ERROR;
 }
 
@@ -1306,14 +1323,14 @@ ft_error ftx_rerandomise(ft_ge25519_array c1, ft_ge25519_array c2, const uint8_t
 {
     ENSURE_INIT();
     if (c1->n != n || c2->n != n) return FT_ERR_SIZE_MISMATCH;
-    const uint32_t *tab;
-    ft_error err = ensure_pk_table(pk, &tab);
+    const ft::CombTable *tab;
+    ft_error err = ensure_pk_table(pk, n, &tab);
     if (err) return err;
     if (n == 0) return FT_ERR_NO_ERROR;
     void *s;
     CK(scratch(&s, align256(n * 32)));
     CK(h2d(s, r, n * 32));
-    CK(ft::rerandomise(ft::view_of(c1), ft::view_of(c2), n, (const uint8_t *)s, tab, g.stream));
+    CK(ft::rerandomise(ft::view_of(c1), ft::view_of(c2), n, (const uint8_t *)s, g.b, *tab, g.d_fault, g.stream));
     return FT_ERR_NO_ERROR;
 }
 
@@ -1467,24 +1484,27 @@ namespace ft {
 
 cudaMemPool_t host_pool() { return g.pool; }
 
-// encryption tables of a public key for a server (cudaMalloc'd; the server
-// frees them)
-ft_error ftx_server_pk_table(const uint8_t *pk, uint32_t **table)
+const CombTable &base_table() { return g.b; }
+
+int *fault_word() { return g.d_fault; }
+
+// the tables of a public key for a server (cudaMalloc'd; the server frees them)
+ft_error ftx_server_pk_table(const uint8_t *pk, CombTable *table)
 {
-    *table = nullptr;
-    cudaError_t e = cudaMalloc((void **)table, ENC_TABLES_BYTES);
+    cudaError_t e = cudaMalloc((void **)&table->mem, COMB_TABLE_BYTES);
     if (e != cudaSuccess) {
-        *table = nullptr;
+        table->mem = nullptr;
         return map_err(e);
     }
-    ft_error err = build_key_tables(*table, pk);
+    ft_error err = build_key_table(*table, pk);
     if (!err) {
-        e = cudaStreamSynchronize(g.stream);
+        e = comb_t256(*table, g.stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(g.stream);
         if (e != cudaSuccess) err = map_err(e);
     }
     if (err) {
-        cudaFree(*table);
-        *table = nullptr;
+        cudaFree(table->mem);
+        table->mem = nullptr;
     }
     return err;
 }

@@ -104,23 +104,36 @@ cudaError_t validate(View v, size_t n, long long *d_bad, cudaStream_t st);
 // ---- scalar multiplication (k_smul.cu)
 // per-element (sc_step = 1) or broadcast (sc_step = 0) 32-byte scalars
 cudaError_t smul_var(View v, size_t n, const uint8_t *d_scalars, int sc_step, cudaStream_t st);
-// a_i * B by the radix-32 comb over B's table (btab, ENC_TABLE_WORDS words)
-cudaError_t smul_base(View v, size_t n, const uint8_t *d_scalars, int sc_step, const uint32_t *btab, cudaStream_t st);
-cudaError_t smul_base_small(View v, size_t n, const uint64_t *d_small, const uint32_t *btab, cudaStream_t st);
-// ---- fixed-base products (k_encrypt.cu): the radix-32 comb (enc_comb.cuh)
-// over tables of (j+1) * 32^row * Q, j < ENC_ENTRIES, row < ENC_ROWS (affine,
-// 24 words per entry); the encryption tables are B's followed by PK's
-constexpr size_t ENC_TABLE_WORDS = (size_t)ENC_ROWS * ENC_ENTRIES * 24;
-constexpr size_t ENC_TABLES_BYTES = 2 * ENC_TABLE_WORDS * 4;
-// the table of the point at element 0 of q
-cudaError_t build_enc_table(uint32_t *d_table, View q, cudaStream_t st);
-// c1 = r*B, c2 = m*B + r*PK
+// ---- fixed-base products (k_encrypt.cu): combs in radix 32 (short arrays) and
+// radix 256 over tables of a point, COMB_TABLE_BYTES of device memory, 16-byte
+// aligned.  comb_bases fills the base points both tables are made of; a
+// launch over `units` products reads the radix-256 table where
+// comb_is_wide(units), the radix-32 table elsewhere.
+constexpr size_t COMB_TABLE_BYTES = (52 + 32) * 128 + (size_t)16 * 6 * 64 * 16 + (size_t)32 * 16 * 1280;
+struct CombTable {
+    uint8_t *mem = nullptr;
+};
+// B's tables and the fault word of the library (ft_api.cu)
+const CombTable &base_table();
+int *fault_word();
+cudaError_t comb_bases(CombTable t, View q, cudaStream_t st); // Q: element 0 of q
+cudaError_t comb_t32(CombTable t, cudaStream_t st);
+cudaError_t comb_t256(CombTable t, cudaStream_t st);
+bool comb_is_wide(size_t units);
+// (fault: a word that a kernel sets, and nothing clears, when a bounded wait
+// ran out and its results are not valid)
+// a_i * B; sc_step 0: one scalar for all
+cudaError_t smul_base(View v, size_t n, const uint8_t *d_scalars, int sc_step, const CombTable &b, int *fault,
+                      cudaStream_t st);
+cudaError_t smul_base_small(View v, size_t n, const uint64_t *d_small, const CombTable &b, int *fault, cudaStream_t st);
 // ciphertexts one pass of the encryption grid takes (separate arrays)
 size_t encrypt_pass();
-cudaError_t encrypt(View c1, View c2, size_t n, const uint8_t *d_r, const uint64_t *d_m,
-                    int m_digits, const uint32_t *d_tables, cudaStream_t st);
+// c1 = r*B, c2 = m*B + r*PK, m < 2^bits
+cudaError_t encrypt(View c1, View c2, size_t n, const uint8_t *d_r, const uint64_t *d_m, unsigned bits,
+                    const CombTable &b, const CombTable &pk, int *fault, cudaStream_t st);
 // (c1, c2) += (r*B, r*PK): a fresh encryption of zero added in place
-cudaError_t rerandomise(View c1, View c2, size_t n, const uint8_t *d_r, const uint32_t *d_tables, cudaStream_t st);
+cudaError_t rerandomise(View c1, View c2, size_t n, const uint8_t *d_r, const CombTable &b, const CombTable &pk,
+                        int *fault, cudaStream_t st);
 // discrete-log table of j*B, j < m_max (k_elgamal.cu): open addressing over
 // the canonical encodings, cap slots (a power of two >= 2 m_max)
 struct DlogTable {

@@ -124,7 +124,7 @@ struct ftx_server_s {
     std::map<ft_ge25519_array, size_t> held;
     uint64_t next_ticket = 1;
     bool stop = false;
-    uint32_t *pk_table = nullptr;
+    ft::CombTable pk_table;
     int device = 0;
     std::thread worker;
 
@@ -192,7 +192,7 @@ ft_error ftx_server_s::dispatch(Req *q, Slot &sl)
             x = hm ? cudaMemcpyAsync(dm, hm, r.n * 8, cudaMemcpyHostToDevice, st) : cudaMemsetAsync(dm, 0, r.n * 8, st);
         if (x == cudaSuccess)
             x = ft::encrypt(ft::view_of(a), ft::view_of(b), r.n, (const uint8_t *)dr, (const uint64_t *)dm,
-                            enc_digits(bits), pk_table, st);
+                            bits, ft::base_table(), pk_table, ft::fault_word(), st);
         return x;
     };
     switch (r.op) {
@@ -207,7 +207,8 @@ ft_error ftx_server_s::dispatch(Req *q, Slot &sl)
         e = alloc_on(q, &dr, r.n * 32, st);
         if (e == cudaSuccess) e = cudaMemcpyAsync(dr, r.r, r.n * 32, cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess)
-            e = ft::rerandomise(ft::view_of(r.c1), ft::view_of(r.c2), r.n, (const uint8_t *)dr, pk_table, st);
+            e = ft::rerandomise(ft::view_of(r.c1), ft::view_of(r.c2), r.n, (const uint8_t *)dr, ft::base_table(),
+                                pk_table, ft::fault_word(), st);
         q->res.c1 = r.c1;
         q->res.c2 = r.c2;
         break;
@@ -359,7 +360,7 @@ void ftx_server_s::loop()
 }
 
 namespace ft {
-ft_error ftx_server_pk_table(const uint8_t *pk, uint32_t **table); // ft_api.cu
+ft_error ftx_server_pk_table(const uint8_t *pk, CombTable *table); // ft_api.cu
 }
 
 extern "C" {
@@ -505,7 +506,7 @@ void ftx_server_free(ftx_server s)
         }
         delete q;
     }
-    if (s->pk_table) cudaFree(s->pk_table);
+    if (s->pk_table.mem) cudaFree(s->pk_table.mem);
     delete s;
 }
 

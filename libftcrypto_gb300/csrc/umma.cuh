@@ -1,0 +1,124 @@
+// umma.cuh — tcgen05.mma, mbarriers and bulk copies for the kernels that use
+// the tensor cores as an exact table lookup (k_comb256 in k_encrypt.cu).
+//
+// The A operand is in tensor memory, written by the threads that own its rows;
+// B sits in shared memory in the K-major layout without swizzle: core matrices
+// of 8 rows x 16 bytes (128 contiguous bytes); here all rows of one 16-byte
+// column chunk are contiguous, so element (row, k) of an f16 matrix of R rows
+// is at (k / 8) * 16 R + row * 16 + (k % 8) * 2.
+//
+// Every wait is bounded: mbar_wait gives up after a fixed number of polls and
+// says so, and the kernel then leaves its loops, waits (bounded again) for
+// its own copies and frees its tensor memory.
+#pragma once
+#include "tmem.cuh"
+
+namespace ft {
+
+FT_DEV_TM uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+FT_DEV_TM void mbar_init(uint64_t *b, uint32_t count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(b)), "r"(count) : "memory");
+}
+
+FT_DEV_TM void mbar_fence_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+
+// polls until the phase of the given parity has completed; false after
+// MBAR_POLLS polls (each of which the hardware may hold for a while)
+static constexpr int MBAR_POLLS = 1 << 20;
+
+// SLEEP_NS > 0: sleeps in between, for a warp whose polls would take issue
+// slots from warps that compute
+template <int SLEEP_NS = 0>
+FT_DEV_TM bool mbar_wait(uint64_t *b, uint32_t parity)
+{
+    const uint32_t a = smem_addr(b);
+    uint32_t done = 0;
+#pragma unroll 1
+    for (int i = 0; i < MBAR_POLLS && !done; ++i) {
+        if (SLEEP_NS && i) __nanosleep(SLEEP_NS);
+        asm volatile("{\n\t.reg .pred p;\n\t"
+                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(done)
+                     : "r"(a), "r"(parity)
+                     : "memory");
+    }
+    return done != 0;
+}
+
+FT_DEV_TM void mbar_arrive(uint64_t *b)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(b)) : "memory");
+}
+
+// one arrival on b, and `bytes` of bulk copies to come before its phase ends
+FT_DEV_TM void mbar_expect(uint64_t *b, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(b)), "r"(bytes) : "memory");
+}
+
+// `bytes` (a multiple of 16, both addresses 16-byte aligned) from global to
+// shared memory, counted on b
+FT_DEV_TM void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *b)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_addr(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_addr(b))
+                 : "memory");
+}
+
+// shared-memory matrix descriptor: K-major, no swizzle; `lbo` bytes between
+// core matrices along K, `sbo` along the rows
+FT_DEV_TM uint64_t umma_desc(uint32_t addr, uint32_t lbo, uint32_t sbo)
+{
+    return (uint64_t)((addr >> 4) & 0x3fffu) | (uint64_t)((lbo >> 4) & 0x3fffu) << 16 |
+           (uint64_t)((sbo >> 4) & 0x3fffu) << 32 | (uint64_t)1 << 46;
+}
+
+// kind::f16 with f16 operands, both K-major, f32 accumulators: D type at bit
+// 4, N / 8 at 17, M / 16 at 24
+constexpr uint32_t umma_idesc_f16(int m, int n)
+{
+    return 1u << 4 | (uint32_t)(n >> 3) << 17 | (uint32_t)(m >> 4) << 24;
+}
+
+// D (+)= A B, one K = 16 step, A in tensor memory (row m in lane m, two
+// consecutive f16 a column: 8 columns); issued by one thread
+FT_DEV_TM void umma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t idesc, bool accumulate)
+{
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "setp.ne.u32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+                 "r"(a_tmem), "l"(b), "r"(idesc), "r"((uint32_t)accumulate)
+                 : "memory");
+}
+
+// arrives on b when the issuing thread's earlier tcgen05.mma are done
+FT_DEV_TM void umma_commit(uint64_t *b)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(b))
+                 : "memory");
+}
+
+FT_DEV_TM void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+
+FT_DEV_TM void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+// 24 consecutive columns of the thread's lane
+FT_DEV_TM void tmem_ld24(uint32_t ta, float r[24])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%24];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23}, "
+                 "[%25];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=&f"(r[0]), "=&f"(r[1]), "=&f"(r[2]), "=&f"(r[3]), "=&f"(r[4]), "=&f"(r[5]), "=&f"(r[6]),
+                   "=&f"(r[7]), "=&f"(r[8]), "=&f"(r[9]), "=&f"(r[10]), "=&f"(r[11]), "=&f"(r[12]), "=&f"(r[13]),
+                   "=&f"(r[14]), "=&f"(r[15]), "=&f"(r[16]), "=&f"(r[17]), "=&f"(r[18]), "=&f"(r[19]), "=&f"(r[20]),
+                   "=&f"(r[21]), "=&f"(r[22]), "=&f"(r[23])
+                 : "r"(ta), "r"(ta + 8u)
+                 : "memory");
+}
+
+} // namespace ft
