@@ -169,18 +169,14 @@ size_t ladder_wave_points();
 // ---- reductions (k_reduce.cu)
 size_t reduce_scratch_bytes(size_t n);
 cudaError_t reduce(View out, View src, size_t n, void *d_scratch, cudaStream_t st);
-// scan: per-thread sums of scan_level_k(n) points, recursively, down to one
-// block.  16 points per thread where the level fills the GPU (32 and 64
-// measured slower: 1.61, 2.04 against 1.48 ms at 4M points); 4 on the
-// latency-bound lower levels, whose cost is the chain of additions in one
-// thread.
-constexpr size_t SCAN_SMALL_MAX = 1024;
-constexpr size_t scan_level_k(size_t n) { return n > ((size_t)1 << 18) ? 16 : 4; }
+// scan (k_reduce.cu): sums of at least scan_level_k(n) points in scratch, and
+// one total per 128 of them, recursively while more than SCAN_SMALL_MAX
+constexpr size_t SCAN_SMALL_MAX = 512;
+constexpr size_t scan_level_k(size_t n) { return n > ((size_t)1 << 19) ? 16 : n > ((size_t)1 << 18) ? 8 : 4; }
 constexpr size_t scan_scratch_points(size_t n)
 {
-    return n <= SCAN_SMALL_MAX ? 0
-                               : (n + scan_level_k(n) - 1) / scan_level_k(n) +
-                                     scan_scratch_points((n + scan_level_k(n) - 1) / scan_level_k(n));
+    const size_t sums = (n + scan_level_k(n) - 1) / scan_level_k(n), totals = (sums + 127) / 128;
+    return n <= SCAN_SMALL_MAX ? 0 : sums + totals + scan_scratch_points(totals);
 }
 size_t scan_scratch_bytes(size_t n, int m = 1);
 cudaError_t scan(View v, size_t n, int exclusive, void *d_scratch, cudaStream_t st);

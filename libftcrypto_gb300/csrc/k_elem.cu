@@ -207,10 +207,17 @@ __global__ void __launch_bounds__(256) k_scatter_range(uint4 *d, size_t ds, cons
 // the earlier points wait in shared memory (32 bytes per point).
 static constexpr int ZINV_NT = 128;
 
-FT_DEV void load_z(fe &z, uint32_t &zero_mask, const uint4 *p, size_t s, size_t n, size_t i)
+// the Z of point i (1 past n), as loaded
+FT_DEV void load_z(uint4 z[2], const uint4 *p, size_t s, size_t n, size_t i)
 {
-    if (i < n) fe_from_u4(z, p[4 * s + i], p[5 * s + i]);
-    else fe_1(z);
+    z[0] = i < n ? p[4 * s + i] : make_uint4(1u, 0u, 0u, 0u);
+    z[1] = i < n ? p[5 * s + i] : make_uint4(0u, 0u, 0u, 0u);
+}
+
+// 1 in the place of a zero Z, which the mask then tells
+FT_DEV void use_z(fe &z, uint32_t &zero_mask, const uint4 w[2])
+{
+    fe_from_u4(z, w[0], w[1]);
     zero_mask = 0u - (uint32_t)fe_iszero(z);
     fe one;
     fe_1(one);
@@ -249,34 +256,49 @@ __global__ void __launch_bounds__(ZINV_NT) k_zinv(uint4 *out, const uint4 *p, si
     extern __shared__ uint4 pre[]; // [k][2][ZINV_NT]: product of the thread's first k points
     uint4 *my = pre + threadIdx.x;
     const size_t base = ((size_t)blockIdx.x * (ZINV_NT / 32) + (threadIdx.x >> 5)) * 32 * K + (threadIdx.x & 31);
+    // each point's words are loaded a step ahead of their use
     fe acc, z;
     uint32_t zm;
-    load_z(acc, zm, p, s, n, base);
+    uint4 w[2], nx[6];
+    load_z(w, p, s, n, base);
+    use_z(acc, zm, w);
+    if (K > 1) load_z(nx, p, s, n, base + 32);
 #pragma unroll 1
     for (int k = 1; k < K; ++k) {
         my[(2 * k) * ZINV_NT] = u4_lo(acc);
         my[(2 * k + 1) * ZINV_NT] = u4_hi(acc);
-        load_z(z, zm, p, s, n, base + 32 * (size_t)k);
+        use_z(z, zm, nx);
+        if (k + 1 < K) load_z(nx, p, s, n, base + 32 * (size_t)(k + 1));
         fe_mul(acc, acc, z);
     }
+    auto load = [&](int k) {
+        const size_t i = base + 32 * (size_t)k;
+        load_z(nx, p, s, n, i);
+        if (i < n) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) nx[2 + c] = p[c * s + i];
+        }
+    };
+    load(K - 1);
     fe inv;
     fe_inv(inv, acc);
 #pragma unroll 1
     for (int k = K - 1; k >= 0; --k) {
         const size_t i = base + 32 * (size_t)k;
-        load_z(z, zm, p, s, n, i);
-        fe zinv = inv;
+        use_z(z, zm, nx);
+        fe zinv = inv, x, y;
+        fe_from_u4(x, nx[2], nx[3]);
+        fe_from_u4(y, nx[4], nx[5]);
         if (k) {
+            load(k - 1);
             fe q;
             fe_from_u4(q, my[(2 * k) * ZINV_NT], my[(2 * k + 1) * ZINV_NT]);
             fe_mul_x2(zinv, inv, q, inv, inv, z);
         }
-        fe zero, x, y;
+        fe zero;
         fe_0(zero);
         fe_cmov(zinv, zero, zm);
         if (i < n) {
-            fe_from_u4(x, p[0 * s + i], p[1 * s + i]);
-            fe_from_u4(y, p[2 * s + i], p[3 * s + i]);
             fe_mul_x2(x, x, zinv, y, y, zinv);
             Emit::emit(out + Emit::WORDS * i, x, y);
         }

@@ -1,19 +1,18 @@
 // k_reduce.cu — reductions whose combine operator is point addition.
 //
 //   reduce   sum of n points (ft_array_reduce; k_ft_array_reduce,
-//            ftcrypto.cu:1414-1471).  Pass 1: every thread accumulates a
+//            ftcrypto.cu:1414-1471).  Many points: every thread accumulates a
 //            grid-strided subset with one ge_addto (9 multiplications) per
-//            point, then warp-shuffle and block trees leave one partial per
-//            block; pass 2 reduces the partials in one block.  ~1 addition per
+//            point; then, or for few points at once, four lanes per point
+//            (quad.cuh), a block per SM, and one block.  ~1 addition per
 //            input point (the reference's tree does the same count but with
 //            most threads idle at the upper levels and 160-byte AoS loads).
 //   scan     inclusive / exclusive prefix (ft_array_scan / ft_array_prescan;
-//            ftcrypto.cu:1474-1586): per-thread sums of K consecutive points
-//            (16 on levels that fill the GPU, 4 below), an exclusive scan of
-//            those sums by the same routine (one block once at most 1,024
-//            remain), then each thread rescans its K points from its prefix.
-//            ~2 + 2/16 additions per point, one
-//            point-addition site per kernel, no waits between blocks.  Correct
+//            ftcrypto.cu:1474-1586): per-thread sums of K consecutive points,
+//            block-wide scans of those sums, a scan of the blocks' totals that
+//            shifts them, then each thread rescans its K points from its
+//            prefix.  ~2 + 10/K additions per point, no waits between blocks.
+//            Short arrays are scanned by blocks directly.  Correct
 //            for every length (the reference's kernel indexes its tile sums
 //            wrongly above 256 x grid points, ftcrypto.cu:1512).
 //   segsum   out[s] = sum of src[e] (or src[perm[e]]) for e in
@@ -33,50 +32,82 @@
 
 #include "internal.h"
 #include "points.cuh"
+#include "quad.cuh"
 
 namespace ft {
 
-// ------------------------------------------------------------ block trees
+// ------------------------------------------------------------ sums
 
-// sum over the block; the result is valid in thread 0
-template <int NT>
-FT_DEV void block_sum(ge_p3 &acc, uint4 *sm /* (NT/32) * 8 uint4 */)
+// acc += v, a quad of lanes per point (quad.cuh)
+FT_DEV void quad_addto(fe &acc, const fe &v, QuadX &x)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll 1
-    for (int o = 16; o > 0; o >>= 1) {
-        ge_p3 other;
-        shfl_down_p3(other, acc, o);
-        ge_addto(acc, other);
-    }
-    if (NT > 32) {
-        if (lane == 0) sm_st_p3(sm, warp, acc);
-        __syncthreads();
-        if (warp == 0) {
-            if (lane < NT / 32) sm_ld_p3(acc, sm, lane);
-            else ge_p3_0(acc);
-#pragma unroll 1
-            for (int o = (NT / 64 > 0 ? NT / 64 : 1); o > 0; o >>= 1) {
-                ge_p3 other;
-                shfl_down_p3(other, acc, o);
-                ge_addto(acc, other);
-            }
-        }
-    }
+    fe c;
+    quad_cached(c, v, x);
+    quad_add(acc, c, x);
+    quad_p3(acc, x);
 }
 
-// A minimum of one block per SM in the launch bounds lets ptxas take 124
-// registers instead of 106 (still four blocks of 128 threads per SM): the
-// sum of 16,777,216 points 1.539 -> 1.483 ms.  Two points per step (158
-// registers, three blocks per SM) measured 1.546 ms, with 128 registers
-// forced (spills) 1.559 ms.
+// Sums of few points, each block's in out[block]: what a launch costs is its
+// chain of additions, and with four lanes on each an addition takes 3
+// multiplications in sequence instead of 9.
 template <int NT>
-__global__ void __launch_bounds__(NT, 1) k_reduce(const uint4 *p, size_t s, size_t n, uint4 *out, size_t os)
+__global__ void __launch_bounds__(NT) k_reduce_quad(const uint4 *p, size_t s, size_t n, uint4 *out, size_t os)
 {
-    __shared__ uint4 sm[(NT / 32) * 8];
-    ge_p3 acc;
-    const size_t stride = (size_t)gridDim.x * NT;
-    size_t base = (size_t)blockIdx.x * NT;
+    static_assert(NT % 32 == 0 && NT <= 256, "a warp of quads holds the warps' sums");
+    __shared__ uint4 trade[4 * NT], part[NT / 32 * 8];
+    QuadX x(trade, NT);
+    const int l = threadIdx.x & 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const size_t q = threadIdx.x >> 2, stride = (size_t)gridDim.x * (NT / 4);
+    fe acc, v;
+    size_t base = (size_t)blockIdx.x * (NT / 4);
+    quad_ld(acc, p, s, base + q, n, l);
+#pragma unroll 1
+    for (base += stride; base < n; base += stride) {
+        quad_ld(v, p, s, base + q, n, l);
+        quad_addto(acc, v, x);
+    }
+    auto tree = [&](int o) {
+#pragma unroll 1
+        for (; o >= 4; o >>= 1) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v.v[k] = __shfl_down_sync(0xffffffffu, acc.v[k], o);
+            quad_addto(acc, v, x);
+        }
+    };
+    tree(16);
+    if (NT > 32) {
+        if (lane < 4) {
+            part[8 * warp + l] = u4_lo(acc);
+            part[8 * warp + 4 + l] = u4_hi(acc);
+        }
+        __syncthreads();
+        if (warp > 0) return;
+        if (lane < NT / 8) {
+            fe_from_u4(acc, part[8 * (lane >> 2) + l], part[8 * (lane >> 2) + 4 + l]);
+        } else {
+            fe_0(acc);
+            acc.v[0] = l == 1 || l == 2;
+        }
+        tree(NT / 16);
+    }
+    if (threadIdx.x < 4) quad_st(out, os, blockIdx.x, acc, l);
+}
+
+// Sums of many points, 32 per block.  A minimum of one block per SM in the
+// launch bounds lets ptxas take 124 registers instead of 106 (still four
+// blocks of 128 threads per SM): the sum of 16,777,216 points 1.539 -> 1.483
+// ms.  Two points per step (158 registers, three blocks per SM) measured 1.546
+// ms, with 128 registers forced (spills) 1.559 ms.  A block leaves its last
+// 32 sums to k_reduce_quad: summing them here took 16 warps of an SM five
+// more additions each, 29 us of a launch of 8,388,608 points.
+static constexpr int RED_NT = 128, RED_OUT = 32;
+
+__global__ void __launch_bounds__(RED_NT, 1) k_reduce(const uint4 *p, size_t s, size_t n, uint4 *out, size_t os)
+{
+    __shared__ uint4 sm[8 * 64]; // [word][point]
+    ge_p3 acc, x;
+    const size_t stride = (size_t)gridDim.x * RED_NT;
+    size_t base = (size_t)blockIdx.x * RED_NT;
     if (base + threadIdx.x < n) ld_p3(acc, p, s, base + threadIdx.x);
     else ge_p3_0(acc);
     // block-uniform steps with a barrier each: the warps stay on the same
@@ -88,13 +119,24 @@ __global__ void __launch_bounds__(NT, 1) k_reduce(const uint4 *p, size_t s, size
         __syncthreads();
         const size_t i = base + threadIdx.x;
         if (i < n) {
-            ge_p3 x;
             ld_p3(x, p, s, i);
             ge_addto(acc, x);
         }
     }
-    block_sum<NT>(acc, sm);
-    if (threadIdx.x == 0) st_p3(out, os, blockIdx.x, acc);
+    // 128 sums to 64 to 32; the adding warps are on other schedulers in
+    // other blocks
+    const unsigned w = ((threadIdx.x >> 5) + blockIdx.x) & 3u, t = 32 * w + (threadIdx.x & 31);
+#pragma unroll 1
+    for (unsigned half = 64; half >= RED_OUT; half >>= 1) {
+        __syncthreads();
+        if (t >= half && t < 2 * half) st_p3(sm, 64, t - half, acc);
+        __syncthreads();
+        if (t < half) {
+            ld_p3(x, sm, 64, t);
+            ge_addto(acc, x);
+        }
+    }
+    if (t < RED_OUT) st_p3(out, os, (size_t)blockIdx.x * RED_OUT + t, acc);
 }
 
 // ------------------------------------------------------------ scan
@@ -114,35 +156,6 @@ FT_DEV void warp_scan_incl(ge_p3 &acc, int width = 32)
     }
 }
 
-// exclusive block scan of x; returns the thread's exclusive prefix.  NT <= 1024.
-template <int NT>
-FT_DEV void block_scan_excl(ge_p3 &ex, const ge_p3 &x, uint4 *sm /* (NT/32) * 8 */)
-{
-    static_assert(NT >= 64 && NT <= 1024 && (NT & (NT - 1)) == 0, "a power-of-two number of warps");
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    ge_p3 incl = x;
-    warp_scan_incl(incl);
-    if (lane == 31) sm_st_p3(sm, warp, incl);
-    __syncthreads();
-    if (warp == 0) {
-        ge_p3 w;
-        if (lane < NT / 32) sm_ld_p3(w, sm, lane);
-        else ge_p3_0(w);
-        warp_scan_incl(w, NT / 32); // the warps' totals: log2(NT/32) levels, not 5
-        ge_p3 wex;
-        shfl_up_p3(wex, w, 1);
-        if (lane == 0) ge_p3_0(wex);
-        __syncwarp();
-        if (lane < NT / 32) sm_st_p3(sm, lane, wex);
-    }
-    __syncthreads();
-    ge_p3 lex;
-    shfl_up_p3(lex, incl, 1);
-    if (lane == 0) ge_p3_0(lex);
-    sm_ld_p3(ex, sm, warp);
-    ge_addto(ex, lex);
-}
-
 // The scan kernels take up to two arrays of one length (the two halves of a
 // ciphertext array, ftx_ct_scan): blockIdx.y selects the array, so both are
 // scanned by the same launches and share the latency-bound lower levels.
@@ -155,19 +168,11 @@ struct ScanSet {
     FT_DEV size_t stride() const { return blockIdx.y ? s[1] : s[0]; }
 };
 
-// blocks per SM the scan's and the segmented sum's walks are compiled for
-// (__launch_bounds__ minimum; 1 leaves the register count to ptxas).
-// Measured on GB300 for the 2 x 4,194,304-point ciphertext scan: 1.95 ms
-// unconstrained (sums ~152 registers, apply ~184), 2.09 ms at 3 blocks,
-// 2.11 ms at 4 for the sums and 3 for the rescan, 2.68 ms at 4 for both
-// (128 registers, spills); the segmented-sum walk 1.73 ms at 4 blocks
-// (128 registers) against 1.81 ms at 3.
-#ifndef FT_SCAN_SUMS_MINB
-#define FT_SCAN_SUMS_MINB 1
-#endif
-#ifndef FT_SCAN_APPLY_MINB
-#define FT_SCAN_APPLY_MINB 1
-#endif
+// Blocks of 128 threads per SM that the scan's passes and the segmented sum's
+// walk are compiled for (__launch_bounds__ minimum): three for the scan (168
+// registers; four, 128 registers, spill: 2.68 against 1.95 ms for 2 x 4,194,304
+// points), four for the walk (128 registers: 1.73 against 1.81 ms at three).
+static constexpr int SCAN_BLOCKS = 3;
 #ifndef FT_SEG_WALK_MINB
 #define FT_SEG_WALK_MINB 4
 #endif
@@ -218,148 +223,183 @@ static int wave_fit_k(size_t n, int m, const int *ks, int nk, const int *residen
 // pair is added — no registers held for it, 64 KB per block, still three
 // blocks per SM — measured the same for both halves, 1.046 -> 1.062 ms for
 // one array and 1.014 -> 1.064 ms for the prescan.)
-#ifndef FT_WALK_PAIRS
-#define FT_WALK_PAIRS 1
-#endif
-
-// per-thread sums of K consecutive points: ts[t] = sum of p[tK .. tK+K).
-// With FT_WALK_PAIRS the thread loads its points two at a time: the two
-// 16-byte words of a pair fill one 32-byte sector of each plane, which is
-// then read from DRAM once (one point at a time, the sector's second half
-// can be evicted before the next step and read again: 1.29x the
-// algorithmic bytes in the sums, 1.39x in the rescan, measured), and the
-// rescan waits for memory once per two points.  2 x 4,194,304-point
-// ciphertext scan: 2.045 -> 2.020 ms.
-template <int K>
-__global__ void __launch_bounds__(128, FT_SCAN_SUMS_MINB) k_scan_sums(ScanSet in, size_t n, ScanSet ts)
+// per-thread sums of K consecutive points (K even): ts[t] = sum of p[tK ..
+// tK+K).  The thread loads its points two at a time: the two 16-byte words of
+// a pair fill one 32-byte sector of each plane, which is then read from DRAM
+// once (one point at a time, the sector's second half can be evicted before
+// the next step and read again: 1.29x the algorithmic bytes in the sums,
+// 1.39x in the rescan, measured), and the rescan waits for memory once per two
+// points.  2 x 4,194,304-point ciphertext scan: 2.045 -> 2.020 ms.
+__global__ void __launch_bounds__(128, SCAN_BLOCKS) k_scan_sums(ScanSet in, size_t n, int K, ScanSet ts)
 {
     const uint4 *p = in.ptr();
     const size_t s = in.stride();
-    uint4 *tp = ts.ptr();
-    const size_t tss = ts.stride();
-    const size_t nt = (n + K - 1) / K;
-    FT_GRID_LOOP(t, nt)
-    {
-        const size_t e0 = t * K;
-        ge_p3 acc;
-#if FT_WALK_PAIRS
-        static_assert(K % 2 == 0, "pairs of points");
-        ge_p3 x;
-        ld_p3(acc, p, s, e0);
-        if (e0 + 1 < n) {
-            ld_p3(x, p, s, e0 + 1);
-            ge_addto(acc, x);
-        }
-#pragma unroll 1
-        for (int k = 2; k < K; k += 2) {
-            const size_t e = e0 + k;
-            if (e >= n) break;
-            ge_p3 y;
-            ld_p3(x, p, s, e);
-            const bool two = e + 1 < n;
-            if (two) ld_p3(y, p, s, e + 1);
-            ge_addto(acc, x);
-            if (!two) break;
-            ge_addto(acc, y);
-        }
-#else
-        ld_p3(acc, p, s, e0);
-#pragma unroll 1
-        for (int k = 1; k < K; ++k) {
-            const size_t e = e0 + k;
-            if (e >= n) break;
-            ge_p3 x;
-            ld_p3(x, p, s, e);
-            ge_addto(acc, x);
-        }
-#endif
-        st_p3(tp, tss, t, acc);
+    const size_t t = (size_t)blockIdx.x * 128 + threadIdx.x, e0 = t * K;
+    if (e0 >= n) return;
+    ge_p3 acc, x;
+    ld_p3(acc, p, s, e0);
+    if (e0 + 1 < n) {
+        ld_p3(x, p, s, e0 + 1);
+        ge_addto(acc, x);
     }
+#pragma unroll 1
+    for (int k = 2; k < K; k += 2) {
+        const size_t e = e0 + k;
+        if (e >= n) break;
+        ge_p3 y;
+        ld_p3(x, p, s, e);
+        const bool two = e + 1 < n;
+        if (two) ld_p3(y, p, s, e + 1);
+        ge_addto(acc, x);
+        if (!two) break;
+        ge_addto(acc, y);
+    }
+    st_p3(ts.ptr(), ts.stride(), t, acc);
 }
 
 // rescan each thread's K points starting from its exclusive prefix ts[t];
 // `exclusive` a template parameter: as a run-time flag the inclusive form
 // needed 210 registers (two blocks per SM) instead of 168 (three)
-template <int K, int exclusive>
-__global__ void __launch_bounds__(128, FT_SCAN_APPLY_MINB) k_scan_apply(ScanSet io, size_t n, ScanSet ts)
+template <int exclusive>
+__global__ void __launch_bounds__(128, SCAN_BLOCKS) k_scan_apply(ScanSet io, size_t n, int K, ScanSet ts)
 {
     uint4 *p = io.ptr();
     const size_t s = io.stride();
-    const uint4 *tp = ts.ptr();
-    const size_t tss = ts.stride();
-    const size_t nt = (n + K - 1) / K;
-    FT_GRID_LOOP(t, nt)
-    {
-        ge_p3 pre;
-        ld_p3(pre, tp, tss, t);
-#if FT_WALK_PAIRS
-        static_assert(K % 2 == 0, "pairs of points");
-#pragma unroll 1
-        for (int k = 0; k < K; k += 2) {
-            const size_t e = t * K + k;
-            if (e >= n) break;
-            ge_p3 x, y;
-            ld_p3(x, p, s, e);
-            const bool two = e + 1 < n;
-            if (two) ld_p3(y, p, s, e + 1);
-            if (exclusive) st_p3(p, s, e, pre);
-            ge_addto(pre, x);
-            if (!exclusive) st_p3(p, s, e, pre);
-            if (!two) break;
-            if (exclusive) st_p3(p, s, e + 1, pre);
-            ge_addto(pre, y);
-            if (!exclusive) st_p3(p, s, e + 1, pre);
-        }
-#else
-#pragma unroll 1
-        for (int k = 0; k < K; ++k) {
-            const size_t e = t * K + k;
-            if (e >= n) break;
-            ge_p3 x;
-            ld_p3(x, p, s, e);
-            if (exclusive) st_p3(p, s, e, pre);
-            ge_addto(pre, x);
-            if (!exclusive) st_p3(p, s, e, pre);
-        }
-#endif
-    }
-}
-
-// one block per array scans n <= NT * kpt points in place: sums of kpt
-// consecutive points per thread, a block-wide exclusive scan of them, then
-// the sequential rescan.  One block is latency-bound, so the points are
-// spread over all NT threads (kpt = ceil(n / NT)): the last level of a
-// 4M-point scan (1,024 points) is a chain of 17 dependent additions instead
-// of 41 with a fixed 16 points per thread (194 us per launch).
-template <int NT>
-__global__ void __launch_bounds__(NT) k_scan_small(ScanSet io, size_t n, int kpt, int exclusive)
-{
-    __shared__ uint4 sm[(NT / 32) * 8];
-    uint4 *p = io.ptr();
-    const size_t s = io.stride();
-    const size_t e0 = (size_t)threadIdx.x * kpt;
-    ge_p3 acc;
-    ge_p3_0(acc);
-    if (e0 < n) ld_p3(acc, p, s, e0);
-#pragma unroll 1
-    for (int k = 1; k < kpt; ++k) {
-        const size_t e = e0 + k;
-        if (e >= n) break;
-        ge_p3 x;
-        ld_p3(x, p, s, e);
-        ge_addto(acc, x);
-    }
+    const size_t t = (size_t)blockIdx.x * 128 + threadIdx.x;
+    if (t * K >= n) return;
     ge_p3 pre;
-    block_scan_excl<NT>(pre, acc, sm);
+    ld_p3(pre, ts.ptr(), ts.stride(), t);
 #pragma unroll 1
-    for (int k = 0; k < kpt; ++k) {
-        const size_t e = e0 + k;
+    for (int k = 0; k < K; k += 2) {
+        const size_t e = t * K + k;
         if (e >= n) break;
-        ge_p3 x;
+        ge_p3 x, y;
         ld_p3(x, p, s, e);
+        const bool two = e + 1 < n;
+        if (two) ld_p3(y, p, s, e + 1);
         if (exclusive) st_p3(p, s, e, pre);
         ge_addto(pre, x);
         if (!exclusive) st_p3(p, s, e, pre);
+        if (!two) break;
+        if (exclusive) st_p3(p, s, e + 1, pre);
+        ge_addto(pre, y);
+        if (!exclusive) st_p3(p, s, e + 1, pre);
+    }
+}
+
+// each block scans its 128 P points in place (P consecutive points per
+// thread; the inclusive form only for P = 1) and writes their total
+__global__ void __launch_bounds__(128, SCAN_BLOCKS) k_scan_block(ScanSet io, size_t n, int P, int inclusive, ScanSet tot)
+{
+    __shared__ uint4 sm[4 * 8];
+    uint4 *p = io.ptr();
+    const size_t s = io.stride();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const size_t e0 = ((size_t)blockIdx.x * 128 + threadIdx.x) * P;
+    ge_p3 incl, v;
+    ge_p3_0(incl);
+    if (e0 < n) ld_p3(incl, p, s, e0);
+#pragma unroll 1
+    for (int k = 1; k < P && e0 + k < n; ++k) {
+        ld_p3(v, p, s, e0 + k);
+        ge_addto(incl, v);
+    }
+    __syncwarp();
+    warp_scan_incl(incl);
+    if (lane == 31) sm_st_p3(sm, warp, incl);
+    __syncthreads();
+    if (warp == 0) {
+        if (lane < 4) sm_ld_p3(v, sm, lane);
+        else ge_p3_0(v);
+        warp_scan_incl(v, 4);
+        if (lane == 3) st_p3(tot.ptr(), tot.stride(), blockIdx.x, v);
+        ge_p3 ex;
+        shfl_up_p3(ex, v, 1);
+        if (lane == 0) ge_p3_0(ex);
+        if (lane < 4) sm_st_p3(sm, lane, ex);
+    }
+    if (!inclusive) {
+        shfl_up_p3(v, incl, 1);
+        if (lane == 0) ge_p3_0(v);
+        incl = v;
+    }
+    __syncthreads();
+    sm_ld_p3(v, sm, warp);
+    ge_addto(incl, v); // the block's points before this thread's (and its own)
+#pragma unroll 1
+    for (int k = 0; k < P; ++k) {
+        const size_t e = e0 + k;
+        if (e >= n) break;
+        if (k + 1 < P) ld_p3(v, p, s, e);
+        st_p3(p, s, e, incl);
+        if (k + 1 < P) ge_addto(incl, v);
+    }
+}
+
+// p[e] += the exclusive prefix of e's block of `per` points (a multiple of
+// 128); the first block's is the identity
+__global__ void __launch_bounds__(128) k_scan_shift(ScanSet io, size_t n, int per, ScanSet tot)
+{
+    uint4 *p = io.ptr();
+    const size_t s = io.stride();
+    const size_t e = (size_t)per + (size_t)blockIdx.x * 128 + threadIdx.x;
+    if (e >= n) return;
+    ge_p3 x, y;
+    ld_p3(y, tot.ptr(), tot.stride(), e / per);
+    ld_p3(x, p, s, e);
+    ge_addto(x, y);
+    st_p3(p, s, e, x);
+}
+
+// One block per array scans n <= NT / 4 * kpt points in place, a quad of lanes
+// per addition (quad.cuh): sums of kpt consecutive points per quad, a scan of
+// those over the block, then the rescan.  One block is all latency: 218 points
+// took 52 us with a thread per addition.
+template <int NT>
+__global__ void __launch_bounds__(NT) k_scan_small(ScanSet io, size_t n, int kpt, int exclusive)
+{
+    __shared__ uint4 trade[4 * NT], vals[4 * NT];
+    QuadX x(trade, NT);
+    uint4 *p = io.ptr();
+    const size_t s = io.stride();
+    const int l = threadIdx.x & 3, q = threadIdx.x >> 2;
+    const size_t e0 = (size_t)q * kpt;
+    fe acc, v;
+    quad_ld(acc, p, s, e0, n, l);
+#pragma unroll 1
+    for (int k = 1; k < kpt; ++k) {
+        quad_ld(v, p, s, e0 + k, n, l);
+        quad_addto(acc, v, x);
+    }
+    // inclusive scan over the quads, then the one before; two buffers in turn
+    int flip = 0;
+#pragma unroll 1
+    for (int o = 1;; o <<= 1) {
+        const int back = o < NT / 4 ? o : 1;
+        uint4 *w = vals + flip + threadIdx.x;
+        w[0] = u4_lo(acc);
+        w[NT] = u4_hi(acc);
+        __syncthreads();
+        if (q >= back) {
+            fe_from_u4(v, w[-4 * back], w[NT - 4 * back]);
+        } else {
+            fe_0(v);
+            v.v[0] = l == 1 || l == 2;
+        }
+        __syncwarp();
+        if (o >= NT / 4) break;
+        quad_addto(acc, v, x);
+        flip ^= 2 * NT;
+    }
+    acc = v;
+#pragma unroll 1
+    for (int k = 0; k < kpt; ++k) {
+        const size_t e = e0 + k;
+        quad_ld(v, p, s, e, n, l);
+        if (exclusive && e < n) quad_st(p, s, e, acc, l);
+        __syncwarp();
+        quad_addto(acc, v, x);
+        if (!exclusive && e < n) quad_st(p, s, e, acc, l);
     }
 }
 
@@ -367,12 +407,29 @@ static const int SMALL_NT = 256;
 
 size_t scan_scratch_bytes(size_t n, int m) { return (size_t)m * scan_scratch_points(n) * 128 + 256; }
 
-// thread sums of K = scan_level_k(n) points, an exclusive scan of those sums
-// (the same routine on arrays K times shorter, until one block suffices),
-// then the rescan: about 2 + 2/K additions per point, no waits between blocks.
-// At 4M points the lower levels (262,144 points down to 4,096) take 4 points
-// per thread: 16 made each of their launches a 16-addition chain in
-// under-filled waves (~60 us each).  m arrays (1 or 2) of n points each go
+// Points per thread of the sums and the rescan; 1: the block scans take the
+// points themselves.  Two warps per scheduler hold m * n = 256 points per SM;
+// beyond, K is the least that makes the launches whole waves of SCAN_BLOCKS
+// blocks per SM, up to 80 points a thread (the passes' own time hardly depends
+// on K: 2 x 4,194,304 points 1.84 to 1.91 ms for 16 to 36; the fewer sums, the
+// less the levels below them).
+static int scan_points(size_t n, int m)
+{
+    const size_t sm = (size_t)sm_count(), wave = 128 * SCAN_BLOCKS * sm;
+    if (n * m <= 256 * sm) return 1;
+    size_t waves = (n * m + 80 * wave - 1) / (80 * wave);
+    size_t k = (n * m + waves * wave - 1) / (waves * wave);
+    k = (std::max(k, scan_level_k(n)) + 1) / 2 * 2;
+    return (int)k;
+}
+
+// Sums of K points per thread, block-wide scans of those sums, a scan of the
+// blocks' totals (one block up to SCAN_SMALL_MAX, else this routine), which
+// shifts the sums' scans, then the rescan from each thread's prefix: about
+// 2 + 10 / K additions per point, no waits between blocks.  The chain of
+// additions between the sums and the rescan, which no launch fills the GPU
+// with, is 11 + 13 of a quad + 1 (1,000,000 ciphertexts: 70 us; 156 us as three
+// levels of 4 points per thread and a last block).  m arrays (1 or 2) of n points each go
 // through the same launches; scratch holds m x scan_scratch_points(n) points.
 cudaError_t scan_set(const View *v, int m, size_t n, int exclusive, void *scratch, cudaStream_t st)
 {
@@ -384,34 +441,46 @@ cudaError_t scan_set(const View *v, int m, size_t n, int exclusive, void *scratc
         io.s[i] = v[i].s;
     }
     if (n <= SCAN_SMALL_MAX) {
-        const int kpt = (int)((n + SMALL_NT - 1) / SMALL_NT);
+        const int kpt = (int)((n + SMALL_NT / 4 - 1) / (SMALL_NT / 4));
         k_scan_small<SMALL_NT><<<dim3(1, m), SMALL_NT, 0, st>>>(io, n, kpt, exclusive);
         return cudaGetLastError();
     }
-    // points per thread: 16 above 2^18 points, 4 on the latency-bound lower
-    // levels.  (Choosing 16, 18 or 20 by how well the last wave fills, as
-    // the segmented walk does, measured 7% slower: at 18 and 20 points the
-    // sums pass takes 170 registers and two blocks per SM instead of three.)
-    const size_t K = scan_level_k(n);
+    uint4 *next = (uint4 *)scratch;
+    auto take = [&](ScanSet &set, View *views, size_t count) {
+        for (int i = 0; i < m; ++i) {
+            views[i] = View{next, count};
+            set.p[i] = next;
+            set.s[i] = count;
+            next += FT_PLANES * count;
+        }
+    };
+    const int K = scan_points(n, m);
     const size_t nt = (n + K - 1) / K;
-    View ts[2];
-    ScanSet tset{};
-    for (int i = 0; i < m; ++i) {
-        ts[i] = View{(uint4 *)scratch + (size_t)i * FT_PLANES * nt, nt};
-        tset.p[i] = ts[i].p;
-        tset.s[i] = nt;
-    }
-    void *rest = (uint4 *)scratch + (size_t)m * FT_PLANES * nt;
+    ScanSet sums = io, totals{};
+    View vs[2], vt[2];
     const dim3 grid((unsigned)((nt + 127) / 128), m);
-    if (K == 16) k_scan_sums<16><<<grid, 128, 0, st>>>(io, n, tset);
-    else k_scan_sums<4><<<grid, 128, 0, st>>>(io, n, tset);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    if ((e = scan_set(ts, m, nt, 1, rest, st)) != cudaSuccess) return e;
-    if (K == 16 && exclusive) k_scan_apply<16, 1><<<grid, 128, 0, st>>>(io, n, tset);
-    else if (K == 16) k_scan_apply<16, 0><<<grid, 128, 0, st>>>(io, n, tset);
-    else if (exclusive) k_scan_apply<4, 1><<<grid, 128, 0, st>>>(io, n, tset);
-    else k_scan_apply<4, 0><<<grid, 128, 0, st>>>(io, n, tset);
+    cudaError_t e;
+    if (K > 1) {
+        take(sums, vs, nt);
+        k_scan_sums<<<grid, 128, 0, st>>>(io, n, K, sums);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    // points per thread of the block scans: P (2 + 7 / P additions a point, in
+    // a chain of 2 P + 7): more of them where the chain is not what counts
+    const size_t warps = 128 * (size_t)sm_count(); // threads, one warp per scheduler
+    const int P = K == 1 || nt * m <= warps ? 1 : nt * m <= 4 * warps ? 2 : 4, per = 128 * P;
+    const size_t nb = (nt + per - 1) / per;
+    take(totals, vt, nb);
+    k_scan_block<<<dim3((unsigned)nb, m), 128, 0, st>>>(sums, nt, P, K == 1 && !exclusive, totals);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (nb > 1) {
+        if ((e = scan_set(vt, m, nb, 1, next, st)) != cudaSuccess) return e;
+        k_scan_shift<<<dim3((unsigned)((nt - per + 127) / 128), m), 128, 0, st>>>(sums, nt, per, totals);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    if (K == 1) return cudaSuccess;
+    if (exclusive) k_scan_apply<1><<<grid, 128, 0, st>>>(io, n, K, sums);
+    else k_scan_apply<0><<<grid, 128, 0, st>>>(io, n, K, sums);
     return cudaGetLastError();
 }
 
@@ -422,33 +491,50 @@ cudaError_t scan(View v, size_t n, int exclusive, void *scratch, cudaStream_t st
 
 // ------------------------------------------------------------ reduce launcher
 
-static const int RED_NT = 128;
-
-static unsigned reduce_grid(size_t n)
+// blocks of the first pass over many points: one wave, every block resident
+static size_t reduce_blocks()
 {
-    // one wave of the first pass: every block resident at once
     static std::once_flag once;
     static size_t resident;
-    std::call_once(once, [] { resident = (size_t)resident_blocks((const void *)k_reduce<RED_NT>, RED_NT); });
-    size_t need = (n + RED_NT - 1) / RED_NT;
-    return (unsigned)(need < resident ? (need ? need : 1) : resident);
+    std::call_once(once, [] { resident = (size_t)resident_blocks((const void *)k_reduce, RED_NT); });
+    return resident;
 }
 
-size_t reduce_scratch_bytes(size_t n) { return (size_t)reduce_grid(n) * 128 + 256; }
+// blocks of a quad pass: 32 quads each, up to one per SM
+static size_t quad_blocks(size_t n) { return std::min<size_t>((n + 31) / 32, (size_t)sm_count()); }
 
+size_t reduce_scratch_bytes(size_t n)
+{
+    (void)n;
+    return (reduce_blocks() * RED_OUT + (size_t)sm_count()) * 128 + 256;
+}
+
+// A point per thread of the first pass and more: that pass, whose sums
+// (19,456 with 152 SMs) are then the points; the sums of a block per SM by
+// quads; one block's.  8,388,608 points 780 -> 735 us, 1,000 points 38 -> 15.
 cudaError_t reduce(View out, View src, size_t n, void *scratch, cudaStream_t st)
 {
-    unsigned g = reduce_grid(n);
     if (n == 0) return set_zero(out, 1, st);
-    if (g == 1) {
-        k_reduce<RED_NT><<<1, RED_NT, 0, st>>>(src.p, src.s, n, out.p, out.s);
-        return cudaGetLastError();
+    cudaError_t e;
+    const size_t g = reduce_blocks();
+    uint4 *next = (uint4 *)scratch;
+    if (n > g * RED_NT) {
+        const View part{next, g * RED_OUT};
+        next += FT_PLANES * g * RED_OUT;
+        k_reduce<<<(unsigned)g, RED_NT, 0, st>>>(src.p, src.s, n, part.p, part.s);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        src = part;
+        n = g * RED_OUT;
     }
-    View part{(uint4 *)scratch, g};
-    k_reduce<RED_NT><<<g, RED_NT, 0, st>>>(src.p, src.s, n, part.p, part.s);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_reduce<RED_NT><<<1, RED_NT, 0, st>>>(part.p, part.s, g, out.p, out.s);
+    const size_t q = quad_blocks(n);
+    if (q > 1) {
+        const View part{next, q};
+        k_reduce_quad<128><<<(unsigned)q, 128, 0, st>>>(src.p, src.s, n, part.p, part.s);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        src = part;
+        n = q;
+    }
+    k_reduce_quad<256><<<1, 256, 0, st>>>(src.p, src.s, n, out.p, out.s);
     return cudaGetLastError();
 }
 
