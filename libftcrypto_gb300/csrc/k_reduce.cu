@@ -97,32 +97,46 @@ __global__ void __launch_bounds__(NT) k_reduce_quad(const uint4 *p, size_t s, si
 // launch bounds lets ptxas take 124 registers instead of 106 (still four
 // blocks of 128 threads per SM): the sum of 16,777,216 points 1.539 -> 1.483
 // ms.  Two points per step (158 registers, three blocks per SM) measured 1.546
-// ms, with 128 registers forced (spills) 1.559 ms.  A block leaves its last
+// ms, with 128 registers forced (spills) 1.559 ms.  The next point arrives in
+// shared memory while this one is added (8,388,608 points 749 -> 725 us).  A block leaves its last
 // 32 sums to k_reduce_quad: summing them here took 16 warps of an SM five
 // more additions each, 29 us of a launch of 8,388,608 points.
 static constexpr int RED_NT = 128, RED_OUT = 32;
 
 __global__ void __launch_bounds__(RED_NT, 1) k_reduce(const uint4 *p, size_t s, size_t n, uint4 *out, size_t os)
 {
-    __shared__ uint4 sm[8 * 64]; // [word][point]
+    __shared__ uint4 sm[2 * 8 * RED_NT]; // the next point and this one
     ge_p3 acc, x;
     const size_t stride = (size_t)gridDim.x * RED_NT;
-    size_t base = (size_t)blockIdx.x * RED_NT;
-    if (base + threadIdx.x < n) ld_p3(acc, p, s, base + threadIdx.x);
+    size_t i = (size_t)blockIdx.x * RED_NT + threadIdx.x;
+    uint4 *slot = sm + threadIdx.x, *next = slot + 8 * RED_NT;
+    if (i < n) ld_p3(acc, p, s, i);
     else ge_p3_0(acc);
+    size_t base = (size_t)blockIdx.x * RED_NT + stride;
+    i += stride;
+    if (i < n) point_fetch(slot, RED_NT, p, s, i);
+    points_sent();
     // block-uniform steps with a barrier each: the warps stay on the same
     // stretch of the addition's code and share the instruction caches
     // (instruction-fetch stalls were 0.75 per issue): 2.09 -> 2.01 ms for
     // 16,777,216 points
 #pragma unroll 1
-    for (base += stride; base < n; base += stride) {
+    for (; base < n; base += stride) {
         __syncthreads();
-        const size_t i = base + threadIdx.x;
-        if (i < n) {
-            ld_p3(x, p, s, i);
+        const bool here = i < n;
+        i += stride;
+        if (i < n) point_fetch(next, RED_NT, p, s, i);
+        points_sent();
+        points_wait<1>();
+        if (here) {
+            ld_p3(x, slot, RED_NT, 0);
             ge_addto(acc, x);
         }
+        uint4 *const t = slot;
+        slot = next;
+        next = t;
     }
+    points_wait<0>();
     // 128 sums to 64 to 32; the adding warps are on other schedulers in
     // other blocks
     const unsigned w = ((threadIdx.x >> 5) + blockIdx.x) & 3u, t = 32 * w + (threadIdx.x & 31);
@@ -223,38 +237,39 @@ static int wave_fit_k(size_t n, int m, const int *ks, int nk, const int *residen
 // pair is added — no registers held for it, 64 KB per block, still three
 // blocks per SM — measured the same for both halves, 1.046 -> 1.062 ms for
 // one array and 1.014 -> 1.064 ms for the prescan.)
-// per-thread sums of K consecutive points (K even): ts[t] = sum of p[tK ..
-// tK+K).  The thread loads its points two at a time: the two 16-byte words of
-// a pair fill one 32-byte sector of each plane, which is then read from DRAM
-// once (one point at a time, the sector's second half can be evicted before
-// the next step and read again: 1.29x the algorithmic bytes in the sums,
-// 1.39x in the rescan, measured), and the rescan waits for memory once per two
-// points.  2 x 4,194,304-point ciphertext scan: 2.045 -> 2.020 ms.
+// per-thread sums of K consecutive points: ts[t] = sum of p[tK .. tK+K).  The
+// thread loads its points two at a time: the two 16-byte words of a pair fill
+// one 32-byte sector of each plane, which is then read from DRAM once (one
+// point at a time, the sector's second half can be evicted before the next
+// step and read again: 1.29x the algorithmic bytes in the sums, 1.39x in the
+// rescan, measured), and memory is waited for once per two points.  A step is
+// one addition, with a barrier, so that the block's warps share the
+// instruction caches: 2 x 4,194,304 points 1.80 -> 1.71 ms against two
+// additions a step without.  (Fetching the next pair into shared memory
+// meanwhile measured 1.85 ms, a warp fetching its threads' next four points
+// together, coalesced, 1.79: the additions bound the passes, not the loads.)
 __global__ void __launch_bounds__(128, SCAN_BLOCKS) k_scan_sums(ScanSet in, size_t n, int K, ScanSet ts)
 {
     const uint4 *p = in.ptr();
     const size_t s = in.stride();
     const size_t t = (size_t)blockIdx.x * 128 + threadIdx.x, e0 = t * K;
-    if (e0 >= n) return;
-    ge_p3 acc, x;
-    ld_p3(acc, p, s, e0);
-    if (e0 + 1 < n) {
-        ld_p3(x, p, s, e0 + 1);
-        ge_addto(acc, x);
-    }
+    ge_p3 acc, x, y;
+    if (e0 < n) ld_p3(acc, p, s, e0);
+    if (e0 + 1 < n) ld_p3(y, p, s, e0 + 1);
 #pragma unroll 1
-    for (int k = 2; k < K; k += 2) {
+    for (int k = 1; k < K; ++k) {
+        __syncthreads();
         const size_t e = e0 + k;
-        if (e >= n) break;
-        ge_p3 y;
-        ld_p3(x, p, s, e);
-        const bool two = e + 1 < n;
-        if (two) ld_p3(y, p, s, e + 1);
+        if (e >= n) continue;
+        if (k & 1) {
+            x = y;
+        } else {
+            ld_p3(x, p, s, e);
+            if (e + 1 < n) ld_p3(y, p, s, e + 1);
+        }
         ge_addto(acc, x);
-        if (!two) break;
-        ge_addto(acc, y);
     }
-    st_p3(ts.ptr(), ts.stride(), t, acc);
+    if (e0 < n) st_p3(ts.ptr(), ts.stride(), t, acc);
 }
 
 // rescan each thread's K points starting from its exclusive prefix ts[t];
@@ -265,25 +280,23 @@ __global__ void __launch_bounds__(128, SCAN_BLOCKS) k_scan_apply(ScanSet io, siz
 {
     uint4 *p = io.ptr();
     const size_t s = io.stride();
-    const size_t t = (size_t)blockIdx.x * 128 + threadIdx.x;
-    if (t * K >= n) return;
-    ge_p3 pre;
-    ld_p3(pre, ts.ptr(), ts.stride(), t);
+    const size_t t = (size_t)blockIdx.x * 128 + threadIdx.x, e0 = t * K;
+    ge_p3 pre, x, y;
+    if (e0 < n) ld_p3(pre, ts.ptr(), ts.stride(), t);
 #pragma unroll 1
-    for (int k = 0; k < K; k += 2) {
-        const size_t e = t * K + k;
-        if (e >= n) break;
-        ge_p3 x, y;
-        ld_p3(x, p, s, e);
-        const bool two = e + 1 < n;
-        if (two) ld_p3(y, p, s, e + 1);
+    for (int k = 0; k < K; ++k) {
+        __syncthreads();
+        const size_t e = e0 + k;
+        if (e >= n) continue;
+        if (k & 1) {
+            x = y;
+        } else {
+            ld_p3(x, p, s, e);
+            if (e + 1 < n) ld_p3(y, p, s, e + 1);
+        }
         if (exclusive) st_p3(p, s, e, pre);
         ge_addto(pre, x);
         if (!exclusive) st_p3(p, s, e, pre);
-        if (!two) break;
-        if (exclusive) st_p3(p, s, e + 1, pre);
-        ge_addto(pre, y);
-        if (!exclusive) st_p3(p, s, e + 1, pre);
     }
 }
 
@@ -410,14 +423,13 @@ size_t scan_scratch_bytes(size_t n, int m) { return (size_t)m * scan_scratch_poi
 // Points per thread of the sums and the rescan; 1: the block scans take the
 // points themselves.  Two warps per scheduler hold m * n = 256 points per SM;
 // beyond, K is the least that makes the launches whole waves of SCAN_BLOCKS
-// blocks per SM, up to 80 points a thread (the passes' own time hardly depends
-// on K: 2 x 4,194,304 points 1.84 to 1.91 ms for 16 to 36; the fewer sums, the
-// less the levels below them).
+// blocks per SM, up to 40 points a thread (2 x 4,194,304 points: 1.82 ms at 16,
+// 1.71 at 36, 1.79 at 72; 2 x 1,000,000: 0.53, 0.50, 0.67).
 static int scan_points(size_t n, int m)
 {
     const size_t sm = (size_t)sm_count(), wave = 128 * SCAN_BLOCKS * sm;
     if (n * m <= 256 * sm) return 1;
-    size_t waves = (n * m + 80 * wave - 1) / (80 * wave);
+    size_t waves = (n * m + 40 * wave - 1) / (40 * wave);
     size_t k = (n * m + waves * wave - 1) / (waves * wave);
     k = (std::max(k, scan_level_k(n)) + 1) / 2 * 2;
     return (int)k;

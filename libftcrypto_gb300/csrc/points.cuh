@@ -88,6 +88,27 @@ FT_DEV void sm_ld_p3(ge_p3 &r, const uint4 *sm, int slot)
     fe_from_u4(r.T, q[6], q[7]);
 }
 
+// Points on their way from global memory to shared memory without registers:
+// a thread's slot of point j is 8 uint4, `threads` apart, and is the thread's
+// alone, so points_wait by that thread is all that orders it.
+FT_DEV void point_fetch(uint4 *slot, int threads, const uint4 *p, size_t s, size_t i)
+{
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(slot + k * threads)),
+                     "l"(p + k * s + i)
+                     : "memory");
+}
+
+FT_DEV void points_sent() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+
+// all but the last N groups of this thread's fetches have arrived
+template <int N>
+FT_DEV void points_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // grid-stride loop bounds in size_t
 #define FT_GRID_LOOP(i, n) \
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += (size_t)blockDim.x * gridDim.x)
