@@ -14,7 +14,7 @@
 //   k_validate        k_ft_array_validate (859)
 #include "internal.h"
 #include "points.cuh"
-#include "fe_inv.cuh"
+#include "quad.cuh"
 
 #define FT_TABLE_QUAL static __constant__
 #define FT_WANT_L_SLIDE
@@ -199,8 +199,8 @@ __global__ void __launch_bounds__(256) k_scatter_range(uint4 *d, size_t ds, cons
 // ------------------------------------------------------------ wire formats
 
 // Canonical outputs that divide by Z (folded and affine encodings): K points
-// per thread share one division-step inversion (fe_inv) by Montgomery's
-// trick, 3 multiplications per point more.  A zero Z counts as 1 inside the
+// per thread, four threads, share one division-step inversion (quad_inv) by
+// Montgomery's trick, 3 multiplications per point more.  A zero Z counts as 1 inside the
 // product and its inverse as 0, which is what fe25519_invert(0) = 0 gives
 // the reference.  Thread t of a warp takes the points 32 k + t of the warp's
 // 32 K, so its loads and stores are those of whole warps; the products of
@@ -253,8 +253,8 @@ struct EmitAffine {
 template <class Emit>
 __global__ void __launch_bounds__(ZINV_NT) k_zinv(uint4 *out, const uint4 *p, size_t s, size_t n, int K)
 {
-    extern __shared__ uint4 pre[]; // [k][2][ZINV_NT]: product of the thread's first k points
-    uint4 *my = pre + threadIdx.x;
+    extern __shared__ uint4 pre[]; // [k][2][ZINV_NT]: product of the thread's first k points, k > 0
+    uint4 *my = pre + threadIdx.x - 2 * ZINV_NT;
     const size_t base = ((size_t)blockIdx.x * (ZINV_NT / 32) + (threadIdx.x >> 5)) * 32 * K + (threadIdx.x & 31);
     // each point's words are loaded a step ahead of their use
     fe acc, z;
@@ -280,8 +280,18 @@ __global__ void __launch_bounds__(ZINV_NT) k_zinv(uint4 *out, const uint4 *p, si
         }
     };
     load(K - 1);
-    fe inv;
-    fe_inv(inv, acc);
+    // the quad's four products as one inverse: of this lane's and its
+    // neighbour's, of both pairs', and back
+    fe inv, other;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) other.v[k] = __shfl_xor_sync(0xffffffffu, acc.v[k], 1);
+    fe_mul(inv, acc, other);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) z.v[k] = __shfl_xor_sync(0xffffffffu, inv.v[k], 2);
+    fe_mul(inv, inv, z);
+    fe_mul(other, other, z);
+    quad_inv(inv, inv);
+    fe_mul(inv, inv, other);
 #pragma unroll 1
     for (int k = K - 1; k >= 0; --k) {
         const size_t i = base + 32 * (size_t)k;
@@ -624,7 +634,7 @@ static cudaError_t zinv_launch(uint8_t *o, View v, size_t n, cudaStream_t st)
 {
     if (n == 0) return cudaSuccess;
     const int K = zinv_points(n);
-    const size_t smem = (size_t)K * 2 * ZINV_NT * sizeof(uint4);
+    const size_t smem = (size_t)(K - 1) * 2 * ZINV_NT * sizeof(uint4);
     const unsigned grid = (unsigned)((n + (size_t)ZINV_NT * K - 1) / ((size_t)ZINV_NT * K));
     static SmemAttr attr;
     cudaError_t e = ensure_smem_attr(attr, (const void *)k_zinv<Emit>, (size_t)ZINV_MAX_K * 2 * ZINV_NT * sizeof(uint4));

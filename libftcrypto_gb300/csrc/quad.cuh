@@ -16,6 +16,7 @@
 // lanes of a warp run these together.
 #pragma once
 #include "ge.cuh"
+#include "fe_inv.cuh"
 #include "u4.cuh"
 
 namespace ft {
@@ -148,6 +149,41 @@ FT_DEV void quad_cached(fe &c, const fe &v, QuadX &x)
     quad_yx(t, v, x);
     fe_mul(c, v, fe_d2());
     fe_pick(c, t, c, x.m0);
+}
+
+// 1/z for the z that the four lanes of the quad hold alike (fe_inv): the
+// division steps in all of them, and of the numbers f, g, d and e the one of
+// the lane, 34,300 -> 24,000 cycles
+FT_DEV void quad_inv(fe &out, const fe &z)
+{
+    const int l = threadIdx.x & 3;
+    const uint32_t hi = quad_mask(l, 10), de = quad_mask(l, 12); // g and e; d and e
+    fe c;
+    fe_canon(c, z);
+    int32_t x[INV_LIMBS], y[INV_LIMBS], g[INV_LIMBS];
+    inv_limbs(g, c);
+#pragma unroll
+    for (int i = 0; i < INV_LIMBS; ++i) {
+        const int32_t fg = (int32_t)((uint32_t)inv_p(i) & ~hi) | (int32_t)((uint32_t)g[i] & hi);
+        x[i] = (int32_t)(((uint32_t)fg & ~de) | ((i == 0 ? 1u : 0u) & hi & de));
+    }
+    int32_t eta = -1;
+#pragma unroll 1
+    for (int round = 0; round < INV_ROUNDS; ++round) {
+        const uint32_t w = (uint32_t)x[0] | (uint32_t)x[1] << 30;
+        int32_t u, v, q, r;
+        inv_steps(eta, __shfl_sync(0xffffffffu, w, 0, 4), __shfl_sync(0xffffffffu, w, 1, 4), u, v, q, r);
+        // this lane's row of the matrix, its own number's factor first
+        const int32_t a = (int32_t)(((uint32_t)u & ~hi) | ((uint32_t)r & hi));
+        const int32_t b = (int32_t)(((uint32_t)v & ~hi) | ((uint32_t)q & hi));
+#pragma unroll
+        for (int i = 0; i < INV_LIMBS; ++i) y[i] = __shfl_xor_sync(0xffffffffu, x[i], 1);
+        inv_row(x, x, y, a, b, (int32_t)de);
+    }
+    const int32_t neg = __shfl_sync(0xffffffffu, x[INV_LIMBS - 1], 0, 4) >> 31;
+#pragma unroll
+    for (int i = 0; i < INV_LIMBS; ++i) y[i] = __shfl_sync(0xffffffffu, x[i], 2, 4);
+    inv_finish(out, y, neg);
 }
 
 // the lane's coordinate of point i (identity past n)
