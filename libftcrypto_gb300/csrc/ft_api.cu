@@ -67,6 +67,9 @@ struct Ctx {
     };
     Stage stage[2];
     int stage_next = 0;
+    // streams that ft_mul of short arrays takes in turn (mul_beside)
+    cudaStream_t beside[2] = {nullptr, nullptr};
+    int beside_next = 0;
     // ftx_encrypt's input copies: the first part's on the library stream,
     // the rest's on the transfer stream
     cudaEvent_t in_ev[2] = {nullptr, nullptr};
@@ -166,7 +169,7 @@ cudaError_t d2h(void *dst, const void *src, size_t bytes, cudaStream_t st = null
     return cudaStreamSynchronize(st);
 }
 
-static cudaError_t record_on_stream(cudaEvent_t *ev)
+static cudaError_t record_on_stream(cudaEvent_t *ev, cudaStream_t st)
 {
     if (!*ev) {
         cudaError_t e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
@@ -175,7 +178,7 @@ static cudaError_t record_on_stream(cudaEvent_t *ev)
             return e;
         }
     }
-    return cudaEventRecord(*ev, g.stream);
+    return cudaEventRecord(*ev, st);
 }
 
 // Marks that the work queued so far on the library stream has written a's
@@ -185,21 +188,27 @@ static cudaError_t record_on_stream(cudaEvent_t *ev)
 cudaError_t mark_part(ft_ge25519_array a)
 {
     if (a->exposed.load()) return cudaSuccess;
-    return record_on_stream(&a->part);
+    return record_on_stream(&a->part, g.stream);
 }
 
-// Marks that the work just queued on the library stream completes a's
-// writes: an export of a that follows, with no other use of a in between,
+// Marks that the work just queued on the library stream (or st) completes
+// a's writes: an export of a that follows, with no other use of a in between,
 // waits for this point only (export_begin), not for everything queued after.
 // part_end > 0: the call marked its first part [0, part_end) (mark_part).
-cudaError_t mark_ready(ft_ge25519_array a, size_t part_end = 0)
+cudaError_t mark_ready(ft_ge25519_array a, size_t part_end = 0, cudaStream_t st = nullptr)
 {
     if (a->exposed.load()) return cudaSuccess;
     const uint64_t t = a->touch.load();
-    const cudaError_t e = record_on_stream(&a->ready);
+    const cudaError_t e = record_on_stream(&a->ready, st ? st : g.stream);
     a->ready_touch = e == cudaSuccess ? t : UINT64_MAX; // a failed mark keeps exports in order
     a->part_end = e == cudaSuccess ? part_end : 0;
     return e;
+}
+
+// whether a's last writer marked it and no call has used it since
+bool quiet_since_mark(const_ft_ge25519_array a)
+{
+    return a->ready && !a->exposed.load() && a->touch.load() == a->ready_touch;
 }
 
 // The stream and the device buffer (at least `bytes`) an export of a
@@ -216,8 +225,7 @@ cudaError_t mark_ready(ft_ge25519_array a, size_t part_end = 0)
 cudaError_t export_begin(const_ft_ge25519_array a, size_t bytes, void **buf, cudaStream_t *st, size_t *cut)
 {
     *cut = 0;
-    const bool side = a->ready && !a->exposed.load() && a->touch.load() == a->ready_touch;
-    if (!side) {
+    if (!quiet_since_mark(a)) {
         *st = g.stream;
         return scratch(buf, bytes);
     }
@@ -271,10 +279,10 @@ ft_error export_to_host(uint8_t *mem, const_ft_ge25519_array a, size_t bpp, Conv
 // the transfer stream, so that the copy overlaps kernels already queued on
 // the library stream.  A buffer is refilled only after the kernel that last
 // read it has finished (its `consumed` event, which the caller records after
-// the kernel that reads this copy), and the library stream waits for the
-// copy (`copied`) before that kernel.  The caller waits for `copied` before
+// the kernel that reads this copy), and st, that kernel's stream, waits for
+// the copy (`copied`) before it.  The caller waits for `copied` before
 // returning, so its buffer may be reused at once.
-cudaError_t stage_scalars(void **out, Ctx::Stage **sgp, const void *src, size_t bytes)
+cudaError_t stage_scalars(void **out, Ctx::Stage **sgp, const void *src, size_t bytes, cudaStream_t st)
 {
     Ctx::Stage &sg = g.stage[g.stage_next];
     g.stage_next ^= 1;
@@ -291,7 +299,8 @@ cudaError_t stage_scalars(void **out, Ctx::Stage **sgp, const void *src, size_t 
     }
     if (bytes > sg.cap) {
         // a kernel queued earlier may still read the old buffer: it is freed
-        // in the library stream's order, after that kernel
+        // in the library stream's order, after that kernel (which the library
+        // stream waits for if it is on another)
         if (sg.p) cudaFreeAsync(sg.p, g.stream);
         sg.p = nullptr;
         sg.cap = 0;
@@ -302,7 +311,7 @@ cudaError_t stage_scalars(void **out, Ctx::Stage **sgp, const void *src, size_t 
     if ((e = cudaStreamWaitEvent(g.xfer, sg.consumed, 0)) != cudaSuccess) return e;
     if ((e = cudaMemcpyAsync(sg.p, src, bytes, cudaMemcpyHostToDevice, g.xfer)) != cudaSuccess) return e;
     if ((e = cudaEventRecord(sg.copied, g.xfer)) != cudaSuccess) return e;
-    if ((e = cudaStreamWaitEvent(g.stream, sg.copied, 0)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(st, sg.copied, 0)) != cudaSuccess) return e;
     *out = sg.p;
     *sgp = &sg;
     return cudaSuccess;
@@ -518,6 +527,7 @@ ft_error init_device(int dev)
     int prio_lo = 0, prio_hi = 0;
     CK(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi));
     CK(cudaStreamCreateWithPriority(&g.xfer, cudaStreamNonBlocking, prio_hi));
+    for (auto &st : g.beside) CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     for (auto &ev : g.in_ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     cudaMemPoolProps pp;
     std::memset(&pp, 0, sizeof pp);
@@ -560,6 +570,8 @@ void init_release()
 {
     if (g.stream) cudaStreamSynchronize(g.stream);
     if (g.xfer) cudaStreamSynchronize(g.xfer);
+    for (auto &st : g.beside)
+        if (st) cudaStreamDestroy(st);
     for (auto &sg : g.stage) {
         if (sg.copied) cudaEventDestroy(sg.copied);
         if (sg.consumed) cudaEventDestroy(sg.consumed);
@@ -1014,6 +1026,29 @@ static ft_error neg_impl(ft_ge25519_array array)
 
 void ft_neg(ft_ge25519_array array) { g.last_void = neg_impl(array); }
 
+// ft_mul of a short array that nothing has used since its last writer marked
+// it, scalars pinned: what it has to wait for is that mark only, so it runs on
+// a stream beside the library's, where the multiplications of several short
+// arrays (the halves of a ciphertext array) run at the same time, each of them
+// too short to fill the GPU.  The library's stream waits for it, so whatever
+// is queued there later comes after it as before.
+static ft_error mul_beside(ft_ge25519_array array, const uint8_t *scalars, size_t n)
+{
+    cudaStream_t st = g.beside[g.beside_next];
+    g.beside_next ^= 1;
+    void *s;
+    Ctx::Stage *sg;
+    CK(cudaStreamWaitEvent(st, array->ready, 0));
+    CK(stage_scalars(&s, &sg, scalars, n * 32, st));
+    const cudaError_t e = ft::smul_var(ft::view_of(array), n, (const uint8_t *)s, 1, st);
+    CK(cudaEventRecord(sg->consumed, st));
+    CK(mark_ready(array, 0, st));
+    CK(cudaStreamWaitEvent(g.stream, array->ready, 0));
+    CK(cudaEventSynchronize(sg->copied)); // the caller may reuse its buffer
+    CK(e);
+    return FT_ERR_NO_ERROR;
+}
+
 ft_error ft_mul(ft_ge25519_array array, const uint8_t *scalars, size_t n)
 {
     ENSURE_INIT();
@@ -1021,9 +1056,11 @@ ft_error ft_mul(ft_ge25519_array array, const uint8_t *scalars, size_t n)
     if (n == 0) return FT_ERR_NO_ERROR;
     const void *s;
     Ctx::Stage *sg = nullptr;
-    if (host_is_pinned(scalars)) {
+    const bool pinned = host_is_pinned(scalars);
+    if (pinned && ft::ladder_is_short(n) && quiet_since_mark(array)) return mul_beside(array, scalars, n);
+    if (pinned) {
         void *p;
-        CK(stage_scalars(&p, &sg, scalars, n * 32));
+        CK(stage_scalars(&p, &sg, scalars, n * 32, g.stream));
         s = p;
     } else {
         void *p;

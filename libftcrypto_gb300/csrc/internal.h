@@ -162,6 +162,8 @@ size_t ladder_wave_192();
 size_t ladder_wave_224();
 int ladder_block();
 int set_ladder_block(int nt);
+// whether n products leave most of the GPU idle
+bool ladder_is_short(size_t n);
 // points one wave of the current ladder launch holds (resident blocks x
 // threads), 0 if unknown
 size_t ladder_wave_points();

@@ -119,6 +119,9 @@ size_t ladder_wave_points()
     }
 }
 
+// up to three of the quad kernel's warps per scheduler
+bool ladder_is_short(size_t n) { return g_ladder_nt == 384 && n <= 96 * (size_t)sm_count(); }
+
 static cudaError_t smul_quad(View v, size_t n, const uint4 *sc, int sc_step, cudaStream_t st)
 {
     k_smul_quad<<<(unsigned)((n + QUAD_NT / 4 - 1) / (QUAD_NT / 4)), QUAD_NT, 0, st>>>(v.p, v.s, n, sc, sc_step);

@@ -37,3 +37,38 @@ def test_lengths(ft, pool, n):
     b = base.get_subset(idx)
     b.scale(k[0])
     assert (b.to_packed() == scaled[idx]).all()
+
+
+@pytest.mark.parametrize("n", [1, 33, 96 * SM, 96 * SM + 1])
+def test_short_arrays_at_the_same_time(ft, orc, pool, n):
+    """Short arrays are multiplied beside each other: twice in a row, with the
+    scalars' pinned buffer refilled after each call, a length change and an
+    addition of one to the other in between, exports and a free right after."""
+    torch = pytest.importorskip("torch")
+    pts, k, _, _ = pool
+    i1, i2 = np.arange(n) % len(pts), (np.arange(n) * 5 + 3) % len(pts)
+    hk = torch.empty((n, 32), dtype=torch.uint8).pin_memory().numpy()
+    a, b = ft.Array.from_packed(pts[i1]), ft.Array.from_packed(pts[i2])
+    wa, wb = pts[i1], pts[i2]
+    for turn in range(3):
+        for arr in (a, b):
+            hk[:] = k[(np.arange(n) + 7 * turn + (arr is b)) % len(k)]
+            arr.mul(hk)
+            hk[:] = 255  # the caller's own again
+        wa = orc.mul(wa, k[(np.arange(n) + 7 * turn) % len(k)], threads=8)
+        wb = orc.mul(wb, k[(np.arange(n) + 7 * turn + 1) % len(k)], threads=8)
+        if turn == 1:
+            a.add(b)
+            wa = orc.add(wa, wb, threads=8)
+    c = ft.Array.from_packed(pts[i1])
+    c.add(a)
+    assert (a.to_packed() == wa).all()
+    assert (b.to_packed() == wb).all()
+    hk[:] = k[np.arange(n) % len(k)]
+    b.mul(hk)
+    b.set_length(n // 2)
+    wb = orc.mul(wb, k[np.arange(n) % len(k)], threads=8)
+    assert (b.to_packed() == wb[:n // 2]).all()
+    a.mul(hk)
+    a.free()
+    assert (c.to_packed() == orc.add(pts[i1], wa, threads=8)).all()
