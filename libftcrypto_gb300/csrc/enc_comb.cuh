@@ -1,6 +1,7 @@
-// enc_comb.cuh — the fixed-base comb in signed radix 32 (every fixed-base
-// product of the library: encryption, ft_array_from_scalars,
-// ft_array_from_small_scalars, ft_array_init_scalar).
+// enc_comb.cuh — enc_ref_scalar, the scalar every fixed-base product uses, and
+// the fixed-base comb in signed radix 32 with a masked select, which the
+// kernels' comb in radix 256 (comb256.cuh) took the place of: the host tests
+// still check digits, table entries and products by it.
 //
 // A scalar a < 2^256 is written as ENC_ROWS = 52 digits d_i in [-16, 16):
 // b = a + sum_{i<52} 16 * 32^i (below 2^260), d_i = bits [5i, 5i+5) of b
@@ -71,8 +72,6 @@ FT_DEV void shr5_288(uint32_t c[9])
 static constexpr int ENC_SEL_GROUP = FT_ENC_SEL_GROUP;
 static_assert(ENC_ENTRIES % ENC_SEL_GROUP == 0, "select grouping");
 
-// (S: the stride of the table's words in uint4.)
-template <int S = 1>
 FT_DEV void enc_select(ge_precomp &t, int d, const uint4 *row)
 {
     const uint32_t bneg = (uint32_t)d >> 31;
@@ -87,11 +86,11 @@ FT_DEV void enc_select(ge_precomp &t, int d, const uint4 *row)
     for (int k = 0; k < ENC_ENTRIES; k += ENC_SEL_GROUP) {
 #pragma unroll
         for (int q = 0; q < ENC_SEL_GROUP; ++q) {
-            const uint4 *e = row + 6 * S * (k + q);
+            const uint4 *e = row + 6 * (k + q);
             fe e0, e1, e2;
-            fe_from_u4(e0, e[0 * S], e[1 * S]);
-            fe_from_u4(e1, e[2 * S], e[3 * S]);
-            fe_from_u4(e2, e[4 * S], e[5 * S]);
+            fe_from_u4(e0, e[0], e[1]);
+            fe_from_u4(e1, e[2], e[3]);
+            fe_from_u4(e2, e[4], e[5]);
             const uint32_t m = ct_eq_mask(babs, (uint32_t)(k + q + 1));
 #pragma unroll
             for (int i = 0; i < 8; ++i) {

@@ -34,19 +34,17 @@ struct Ctx {
     long long *d_status = nullptr; // one device word for "last bad index"
     ft_error last_void = FT_ERR_NO_ERROR;
     // comb tables of the last PK_CACHE public keys used, least recently used
-    // replaced: a key's base points are a chain of 255 doublings, so callers
-    // alternating between a few keys build each once; its radix-256 table
-    // waits for the first call long enough to read it
+    // replaced: a key's base points are a chain of 248 doublings, so callers
+    // alternating between a few keys build each once
     struct KeyTab {
         uint8_t pk[32];
         ft::CombTable t;
-        bool wide = false;
         uint64_t used = 0; // 0: empty
     };
     static constexpr int PK_CACHE = 4;
     KeyTab keys[PK_CACHE];
     uint64_t key_clock = 0;
-    ft::CombTable b; // B's tables (fixed-base products)
+    ft::CombTable b; // B's table (fixed-base products)
     // set by a kernel whose bounded wait ran out (mapped host memory): its
     // results are not valid, and every later call reports it
     volatile int *fault = nullptr;
@@ -413,8 +411,8 @@ ft_error status_read(int64_t *res)
     return FT_ERR_NO_ERROR;
 }
 
-// the base points and the radix-32 table of the public key pk (32-byte folded
-// encoding) into t (COMB_TABLE_BYTES), queued on the library stream
+// the table of the public key pk (32-byte folded encoding) into t
+// (COMB_TABLE_BYTES), queued on the library stream
 ft_error build_key_table(ft::CombTable t, const uint8_t *pk)
 {
     ft_ge25519_array q;
@@ -425,18 +423,16 @@ ft_error build_key_table(ft::CombTable t, const uint8_t *pk)
         ft_array_free(q);
         return FT_ERR_INVALID_POINT;
     }
-    cudaError_t e = ft::comb_bases(t, ft::view_of(q), g.stream);
-    if (e == cudaSuccess) e = ft::comb_t32(t, g.stream);
+    const cudaError_t e = ft::comb_table(t, ft::view_of(q), g.stream);
     ft_array_free(q);
     CK(e);
     return FT_ERR_NO_ERROR;
 }
 
-// the tables of pk for a call over n ciphertexts, from the cache or built
-// into its least recently used slot (kernels still queued on the library
-// stream that read the slot's old tables run before the rebuild, in stream
-// order)
-ft_error ensure_pk_table(const uint8_t *pk, size_t n, const ft::CombTable **table)
+// the table of pk, from the cache or built into its least recently used slot
+// (kernels still queued on the library stream that read the slot's old table
+// run before the rebuild, in stream order)
+ft_error ensure_pk_table(const uint8_t *pk, const ft::CombTable **table)
 {
     Ctx::KeyTab *slot = &g.keys[0];
     bool found = false;
@@ -447,17 +443,12 @@ ft_error ensure_pk_table(const uint8_t *pk, size_t n, const ft::CombTable **tabl
     }
     if (!found) {
         slot->used = 0;
-        slot->wide = false;
         if (!slot->t.mem) CK(dev_alloc((void **)&slot->t.mem, ft::COMB_TABLE_BYTES));
         ft_error err = build_key_table(slot->t, pk);
         if (err) return err;
         std::memcpy(slot->pk, pk, 32);
     }
     slot->used = ++g.key_clock;
-    if (!slot->wide && ft::comb_is_wide(2 * n)) {
-        CK(ft::comb_t256(slot->t, g.stream));
-        slot->wide = true;
-    }
     *table = &slot->t;
     return FT_ERR_NO_ERROR;
 }
@@ -520,7 +511,7 @@ const char *ft_error_str(ft_error err)
 
 namespace {
 
-// the library's stream, memory pool, status words and B's comb tables
+// the library's stream, memory pool, status words and B's comb table
 ft_error init_device(int dev)
 {
     CK(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
@@ -545,7 +536,7 @@ ft_error init_device(int dev)
     g.fault = (volatile int *)fault;
     *g.fault = 0;
     CK(cudaHostGetDevicePointer((void **)&g.d_fault, fault, 0));
-    // the comb tables of B, from B's encoding (y = 4/5, x even)
+    // the comb table of B, from B's encoding (y = 4/5, x even)
     uint8_t benc[32];
     std::memset(benc, 0x66, 32);
     benc[0] = 0x58;
@@ -556,9 +547,7 @@ ft_error init_device(int dev)
     uint8_t *d_enc = (uint8_t *)s + align256(FT_PLANES_BYTES_PER_POINT);
     CK(cudaMemcpyAsync(d_enc, benc, 32, cudaMemcpyHostToDevice, g.stream));
     CK(ft::decode(bp, d_enc, 1, g.d_status, g.stream));
-    CK(ft::comb_bases(g.b, bp, g.stream));
-    CK(ft::comb_t32(g.b, g.stream));
-    CK(ft::comb_t256(g.b, g.stream));
+    CK(ft::comb_table(g.b, bp, g.stream));
     CK(cudaStreamSynchronize(g.stream)); // benc is on the stack
     dev_free(s);
     CK(cudaStreamSynchronize(g.stream));
@@ -1237,7 +1226,7 @@ ft_error ftx_encrypt_device(ft_ge25519_array c1, ft_ge25519_array c2, const uint
     if (bits < 1 || bits > 64) return FT_ERR_BAD_SIZE;
     if (c1->n != n || c2->n != n) return FT_ERR_SIZE_MISMATCH;
     const ft::CombTable *tab;
-    ft_error err = ensure_pk_table(pk, n, &tab);
+    ft_error err = ensure_pk_table(pk, &tab);
     if (err) return err;
     CK(ft::encrypt(ft::view_of(c1), ft::view_of(c2), n, d_r, d_m, bits, g.b, *tab, g.d_fault, g.stream));
     CK(mark_ready(c1));
@@ -1298,7 +1287,7 @@ ft_error ftx_encrypt(ft_ge25519_array *c1, ft_ge25519_array *c2, const uint8_t *
     if (too_long(n)) return FT_ERR_OUT_OF_MEMORY;
     // the key's tables first (building them uses the scratch buffer)
     const ft::CombTable *tab;
-    ft_error err = ensure_pk_table(pk, n, &tab);
+    ft_error err = ensure_pk_table(pk, &tab);
     if (err) return err;
     ft_ge25519_array a, b;
     if ((err = arr_new(&a, n))) return err;
@@ -1350,7 +1339,7 @@ ft_error ftx_rerandomise_device(ft_ge25519_array c1, ft_ge25519_array c2, const 
     ENSURE_INIT();
     if (c1->n != n || c2->n != n) return FT_ERR_SIZE_MISMATCH;
     const ft::CombTable *tab;
-    ft_error err = ensure_pk_table(pk, n, &tab);
+    ft_error err = ensure_pk_table(pk, &tab);
     if (err) return err;
     CK(ft::rerandomise(ft::view_of(c1), ft::view_of(c2), n, d_r, g.b, *tab, g.d_fault, g.stream));
     return FT_ERR_NO_ERROR;
@@ -1361,7 +1350,7 @@ ft_error ftx_rerandomise(ft_ge25519_array c1, ft_ge25519_array c2, const uint8_t
     ENSURE_INIT();
     if (c1->n != n || c2->n != n) return FT_ERR_SIZE_MISMATCH;
     const ft::CombTable *tab;
-    ft_error err = ensure_pk_table(pk, n, &tab);
+    ft_error err = ensure_pk_table(pk, &tab);
     if (err) return err;
     if (n == 0) return FT_ERR_NO_ERROR;
     void *s;
@@ -1525,7 +1514,7 @@ const CombTable &base_table() { return g.b; }
 
 int *fault_word() { return g.d_fault; }
 
-// the tables of a public key for a server (cudaMalloc'd; the server frees them)
+// the table of a public key for a server (cudaMalloc'd; the server frees them)
 ft_error ftx_server_pk_table(const uint8_t *pk, CombTable *table)
 {
     cudaError_t e = cudaMalloc((void **)&table->mem, COMB_TABLE_BYTES);
@@ -1535,8 +1524,7 @@ ft_error ftx_server_pk_table(const uint8_t *pk, CombTable *table)
     }
     ft_error err = build_key_table(*table, pk);
     if (!err) {
-        e = comb_t256(*table, g.stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(g.stream);
+        e = cudaStreamSynchronize(g.stream);
         if (e != cudaSuccess) err = map_err(e);
     }
     if (err) {

@@ -104,22 +104,17 @@ cudaError_t validate(View v, size_t n, long long *d_bad, cudaStream_t st);
 // ---- scalar multiplication (k_smul.cu)
 // per-element (sc_step = 1) or broadcast (sc_step = 0) 32-byte scalars
 cudaError_t smul_var(View v, size_t n, const uint8_t *d_scalars, int sc_step, cudaStream_t st);
-// ---- fixed-base products (k_encrypt.cu): combs in radix 32 (short arrays) and
-// radix 256 over tables of a point, COMB_TABLE_BYTES of device memory, 16-byte
-// aligned.  comb_bases fills the base points both tables are made of; a
-// launch over `units` products reads the radix-256 table where
-// comb_is_wide(units), the radix-32 table elsewhere.
-constexpr size_t COMB_TABLE_BYTES = (52 + 32) * 128 + (size_t)16 * 6 * 64 * 16 + (size_t)32 * 16 * 1280;
+// ---- fixed-base products (k_encrypt.cu): the radix-256 comb over the table of
+// a point, COMB_TABLE_BYTES of device memory, 16-byte aligned (32 base points,
+// 32 rows of 16 chunks)
+constexpr size_t COMB_TABLE_BYTES = 32 * 128 + (size_t)32 * 16 * 1280;
 struct CombTable {
     uint8_t *mem = nullptr;
 };
-// B's tables and the fault word of the library (ft_api.cu)
+// B's table and the fault word of the library (ft_api.cu)
 const CombTable &base_table();
 int *fault_word();
-cudaError_t comb_bases(CombTable t, View q, cudaStream_t st); // Q: element 0 of q
-cudaError_t comb_t32(CombTable t, cudaStream_t st);
-cudaError_t comb_t256(CombTable t, cudaStream_t st);
-bool comb_is_wide(size_t units);
+cudaError_t comb_table(CombTable t, View q, cudaStream_t st); // of element 0 of q
 // (fault: a word that a kernel sets, and nothing clears, when a bounded wait
 // ran out and its results are not valid)
 // a_i * B; sc_step 0: one scalar for all

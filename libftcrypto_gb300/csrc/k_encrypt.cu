@@ -11,15 +11,13 @@
 //                ladder here, ftcrypto.cu:895-913)
 //
 // Both are lists of units, a unit being one output point: half 0 or 1 of a
-// ciphertext, or a_i * B.  Two kernels compute them:
-//   k_comb256    radix 256, one thread per unit, table rows looked up by the
-//                tensor cores (comb256.cuh); for lengths that fill the GPU
-//   k_comb_lanes radix 32 (enc_comb.cuh), 8 to 32 lanes per unit that share
-//                its rows and add their sums in a tree; for short arrays
-// and these make a point's tables:
-//   k_comb_bases 32^i * Q and 256^i * Q by one chain of doublings, a quad of
-//                lanes per doubling (quad.cuh)
-//   k_comb_t32, k_comb_t256   the entries of the two combs
+// ciphertext, or a_i * B.  k_comb256 computes them, one thread per unit, in
+// radix 256 with table rows looked up by the tensor cores (comb256.cuh); for
+// short arrays the blocks of a cluster share a unit's rows.  A point's table
+// is made by
+//   k_comb_bases 256^i * Q by one chain of doublings, a quad of lanes per
+//                doubling (quad.cuh)
+//   k_comb_t256  the entries
 #include <algorithm>
 #include <cuda_fp16.h>
 
@@ -35,40 +33,30 @@ namespace ft {
 
 // ------------------------------------------------------------ tables
 
-// memory of a point's tables: 52 + 32 base points (8 uint4 each), the
-// radix-32 table (word w of entry e of row r at (6 e + w) * 64 + r), the
-// radix-256 table (COMB_ROW_BYTES a row)
-static constexpr int T32_ROWS = 64, N_BASES = ENC_ROWS + COMB_ROWS;
-static constexpr size_t BASES_U4 = (size_t)N_BASES * 8, T32_U4 = (size_t)ENC_ENTRIES * 6 * T32_ROWS;
-static_assert(BASES_U4 * 16 + T32_U4 * 16 + (size_t)COMB_ROWS * COMB_ROW_BYTES == COMB_TABLE_BYTES, "table size");
+// memory of a point's table: the base points (8 uint4 each), the rows
+static constexpr size_t BASES_U4 = (size_t)COMB_ROWS * 8;
+static_assert(BASES_U4 * 16 + (size_t)COMB_ROWS * COMB_ROW_BYTES == COMB_TABLE_BYTES, "table size");
 
 static uint4 *bases_of(CombTable t) { return (uint4 *)t.mem; }
-static uint4 *t32_of(CombTable t) { return (uint4 *)t.mem + BASES_U4; }
-static uint8_t *t256_of(CombTable t) { return t.mem + (BASES_U4 + T32_U4) * 16; }
+static uint8_t *rows_of(CombTable t) { return t.mem + BASES_U4 * 16; }
 
-// One warp: Q doubled 255 times, kept every 5 and every 8 bits.  A chain of
-// dependent doublings is all latency; with four lanes on each a doubling
-// takes a squaring and a multiplication in sequence instead of seven.
+// One warp: Q doubled 248 times, kept every 8 bits.  A chain of dependent
+// doublings is all latency; with four lanes on each a doubling takes a
+// squaring and a multiplication in sequence instead of seven.
 __global__ void __launch_bounds__(32) k_comb_bases(uint4 *out, const uint4 *q, size_t qs)
 {
     __shared__ uint4 trade[4 * 32];
     QuadX x(trade, 32);
-    const int l = threadIdx.x & 3;
-    const bool w = threadIdx.x < 4;
+    const int l = threadIdx.x & 3, plane = l == 0 ? 6 : l == 3 ? 0 : 2 * l;
     fe v;
     quad_ld(v, q, qs, 0, 1, l);
-    const int plane = l == 0 ? 6 : l == 3 ? 0 : 2 * l;
 #pragma unroll 1
     for (int bit = 0;; ++bit) {
-        if (w && bit % 5 == 0) {
-            out[(bit / 5) * 8 + plane] = u4_lo(v);
-            out[(bit / 5) * 8 + plane + 1] = u4_hi(v);
+        if (threadIdx.x < 4 && bit % 8 == 0) {
+            out[bit + plane] = u4_lo(v);
+            out[bit + plane + 1] = u4_hi(v);
         }
-        if (w && bit % 8 == 0) {
-            out[(ENC_ROWS + bit / 8) * 8 + plane] = u4_lo(v);
-            out[(ENC_ROWS + bit / 8) * 8 + plane + 1] = u4_hi(v);
-        }
-        if (bit == 5 * (ENC_ROWS - 1)) break;
+        if (bit == 8 * (COMB_ROWS - 1)) break;
         __syncwarp();
         quad_dbl(v, x);
         quad_p3(v, x);
@@ -106,29 +94,13 @@ FT_DEV void comb_entry(ge_precomp &t, const uint4 *base, int k, int bits)
     fe_canon(t.xy2d, t.xy2d);
 }
 
-__global__ void __launch_bounds__(64) k_comb_t32(uint4 *out, const uint4 *bases)
-{
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int row = t % T32_ROWS, e = t / T32_ROWS;
-    if (row >= ENC_ROWS || e >= ENC_ENTRIES) return;
-    ge_precomp p;
-    comb_entry(p, bases + 8 * row, e + 1, 5);
-    uint4 *o = out + (size_t)e * 6 * T32_ROWS + row;
-    o[0 * T32_ROWS] = u4_lo(p.yplusx);
-    o[1 * T32_ROWS] = u4_hi(p.yplusx);
-    o[2 * T32_ROWS] = u4_lo(p.yminusx);
-    o[3 * T32_ROWS] = u4_hi(p.yminusx);
-    o[4 * T32_ROWS] = u4_lo(p.xy2d);
-    o[5 * T32_ROWS] = u4_hi(p.xy2d);
-}
-
 __global__ void __launch_bounds__(64) k_comb_t256(uint8_t *out, const uint4 *bases)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int row = t / COMB_K, k = t % COMB_K;
     if (row >= COMB_ROWS) return;
     ge_precomp p;
-    comb_entry(p, bases + 8 * (ENC_ROWS + row), k + 1, 8);
+    comb_entry(p, bases + 8 * row, k + 1, 8);
     uint8_t *o = out + (size_t)row * COMB_ROW_BYTES;
     auto put = [&](int f, const fe &x) {
 #pragma unroll
@@ -144,21 +116,12 @@ __global__ void __launch_bounds__(64) k_comb_t256(uint8_t *out, const uint4 *bas
     for (int n = 72; n < COMB_N; ++n) *(__half *)(o + comb_offset(n, k)) = __uint2half_rn(0u);
 }
 
-cudaError_t comb_bases(CombTable t, View q, cudaStream_t st)
+cudaError_t comb_table(CombTable t, View q, cudaStream_t st)
 {
     k_comb_bases<<<1, 32, 0, st>>>(bases_of(t), q.p, q.s);
-    return cudaGetLastError();
-}
-
-cudaError_t comb_t32(CombTable t, cudaStream_t st)
-{
-    k_comb_t32<<<T32_ROWS * ENC_ENTRIES / 64, 64, 0, st>>>(t32_of(t), bases_of(t));
-    return cudaGetLastError();
-}
-
-cudaError_t comb_t256(CombTable t, cudaStream_t st)
-{
-    k_comb_t256<<<COMB_ROWS * COMB_K / 64, 64, 0, st>>>(t256_of(t), bases_of(t));
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    k_comb_t256<<<COMB_ROWS * COMB_K / 64, 64, 0, st>>>(rows_of(t), bases_of(t));
     return cudaGetLastError();
 }
 
@@ -166,12 +129,12 @@ cudaError_t comb_t256(CombTable t, cudaStream_t st)
 
 // What a launch computes: for each half h in [h0, h1), dst[h][i] (+)= the sum
 // of the rows of scalar i over table tr[h] (`scalar` set) and of mrows[h]
-// rows of m[i] over tm.  Table pointers are those of the launch's radix.
+// rows of m[i] over tm.
 struct CombJob {
     uint4 *dst[2]; // (the two-element arrays are read with pick: an index would copy them to local memory)
     size_t s[2];
-    const void *tr[2];
-    const void *tm;
+    const uint8_t *tr[2]; // tables' rows
+    const uint8_t *tm;
     const uint4 *sc; // 32-byte scalars, sc_step apart (0: one for all); null: none
     int sc_step;
     const uint64_t *m;
@@ -220,7 +183,8 @@ struct CombSmem {
     static constexpr int NT = 128 * G;
     static constexpr uint32_t A = COMB_N, PER_WG = COMB_N + COMB_K / 2, COLS = G == 1 ? 256 : 512;
     static_assert(G * PER_WG <= COLS, "tensor memory");
-    static constexpr size_t B = 0, DIG = 3 * (size_t)COMB_ROW_BYTES, USED = DIG + (size_t)8 * NT * 4;
+    static constexpr size_t B = 0, DIG = 3 * (size_t)COMB_ROW_BYTES, X = DIG + (size_t)8 * NT * 4;
+    static constexpr size_t USED = X + (G == 1 ? 2 * (size_t)8 * NT * 16 : 0); // X: points from the cluster's others
     static constexpr size_t BYTES = std::max(USED, (size_t)(G == 1 ? 80 : 116) * 1024);
 };
 
@@ -239,8 +203,11 @@ struct CombSmem {
 // warpgroup to be ready issuing (it takes that warp 1,100 cycles, in which its
 // own row and so its warpgroup's next product wait); 5.55 with one warp
 // issuing for all, on whose scheduler the computing warps fell behind.
-template <int G, bool ACC>
-__global__ void __launch_bounds__(128 * (G + 1), 1) k_comb256(CombJob j, int *fault)
+// SPLIT (G = 1): the blocks of a cluster (1, 2, 4 or 8) take a part of a tile's
+// rows each, then add their points up in pairs, through the shared memory of
+// the lower block of each pair.
+template <int G, bool ACC, bool SPLIT>
+__global__ void __launch_bounds__(128 * (G + 1), SPLIT ? 2 : 1) k_comb256(CombJob j, int *fault)
 {
     using S = CombSmem<G>;
     extern __shared__ __align__(128) uint8_t sm[];
@@ -249,6 +216,14 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) k_comb256(CombJob j, int *fa
     const int tid = threadIdx.x, wg = tid >> 7, warp = tid >> 5;
     const int nr = j.sc ? COMB_ROWS : 0;
     const unsigned per_half = (unsigned)((j.n + S::NT - 1) / S::NT), tiles = per_half * (j.h1 - j.h0);
+    const unsigned parts = SPLIT ? cluster_size() : 1u, part = SPLIT ? cluster_rank() : 0u;
+    const unsigned tile0 = blockIdx.x / parts, hop = gridDim.x / parts;
+    // this block's rows [r0, r1) of a tile of half h
+    auto span = [&](int h, int &r0, int &r1) {
+        const unsigned rows = nr + CombJob::pick(j.mrows, h);
+        r0 = (int)(rows * part / parts);
+        r1 = (int)(rows * (part + 1) / parts);
+    };
     if (warp == 0) tmem_alloc(&s_taddr, S::COLS);
     if (tid == 0) {
 #pragma unroll
@@ -264,31 +239,33 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) k_comb256(CombJob j, int *fa
         mbar_fence_init();
     }
     tmem_sync_threads();
+    if (SPLIT) cluster_sync(); // every block of it runs
 
+    ge_p3 h;
     if (wg == G && warp - 4 * G == 3) { // the loads
         if ((tid & 31) == 0) {
-            unsigned tile = blockIdx.x, loads = 0;
-            int t = 0;
+            unsigned loads = 0, buf = 0, use = 0;
             bool bad = false;
 #pragma unroll 1
-            for (unsigned buf = 0, use = 0; tile < tiles && !bad; ++loads) {
+            for (unsigned tile = tile0; tile < tiles && !bad; tile += hop) {
                 const int h = j.h1 - 1 - (int)(tile / per_half);
-                const uint8_t *src = t < nr
-                                         ? (const uint8_t *)CombJob::pick(j.tr, h) + (size_t)(nr - 1 - t) * COMB_ROW_BYTES
-                                         : (const uint8_t *)j.tm + (size_t)(t - nr) * COMB_ROW_BYTES;
-                // the buffer's use before this one
-                if (use && !mbar_wait<COMB_SLEEP>(&empty[buf], (use - 1) & 1)) bad = true;
-                if (!bad) {
+                int r0, r1;
+                span(h, r0, r1);
+#pragma unroll 1
+                for (int t = r0; t < r1; ++t, ++loads) {
+                    const uint8_t *src = t < nr ? CombJob::pick(j.tr, h) + (size_t)(nr - 1 - t) * COMB_ROW_BYTES
+                                                : j.tm + (size_t)(t - nr) * COMB_ROW_BYTES;
+                    // the buffer's use before this one
+                    if (use && !mbar_wait<COMB_SLEEP>(&empty[buf], (use - 1) & 1)) {
+                        bad = true;
+                        break;
+                    }
                     mbar_expect(&full[buf], COMB_ROW_BYTES);
                     bulk_load(sm + S::B + buf * COMB_ROW_BYTES, src, COMB_ROW_BYTES, &full[buf]);
-                }
-                if (++t == nr + CombJob::pick(j.mrows, h)) {
-                    t = 0;
-                    tile += gridDim.x;
-                }
-                if (++buf == 3) {
-                    buf = 0;
-                    ++use;
+                    if (++buf == 3) {
+                        buf = 0;
+                        ++use;
+                    }
                 }
             }
             // the last copies have landed before the block ends
@@ -303,8 +280,11 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) k_comb256(CombJob j, int *fa
         if (g < G && (tid & 31) == 0) {
             unsigned steps = 0;
 #pragma unroll 1
-            for (unsigned k = blockIdx.x; k < tiles; k += gridDim.x)
-                steps += nr + CombJob::pick(j.mrows, j.h1 - 1 - (int)(k / per_half));
+            for (unsigned tile = tile0; tile < tiles; tile += hop) {
+                int r0, r1;
+                span(j.h1 - 1 - (int)(tile / per_half), r0, r1);
+                steps += r1 - r0;
+            }
             const uint32_t dt = s_taddr + S::PER_WG * g;
             unsigned buf = 0, use = 0; // the step's buffer, and that buffer's use
 #pragma unroll 1
@@ -333,18 +313,19 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) k_comb256(CombJob j, int *fa
         unsigned q = 0; // steps so far
         bool bad = false;
 #pragma unroll 1
-        for (unsigned tile = blockIdx.x; tile < tiles && !bad; tile += gridDim.x) {
+        for (unsigned tile = tile0; tile < tiles && !bad; tile += hop) {
             const int half = j.h1 - 1 - (int)(tile / per_half);
             const size_t i = (size_t)(tile % per_half) * S::NT + tid;
             const bool live = i < j.n;
             const int mr = CombJob::pick(j.mrows, half), rows = nr + mr;
-            ge_p3 h;
+            int r0, r1;
+            span(half, r0, r1);
             ge_precomp e;
             int d = 0;
-            // step t adds row t; step -1 only looks up row 0
+            // step t adds row t; the step before r0 only looks up row r0
 #pragma unroll 1
-            for (int t = -1; t < rows; ++t) {
-                if (t >= 0) {
+            for (int t = r0 - 1; t < r1; ++t) {
+                if (t >= r0) {
                     bad = __any_sync(0xffffffffu, !mbar_wait(&done[wg], q & 1));
                     if (bad) break;
                     tmem_fence_after();
@@ -360,8 +341,8 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) k_comb256(CombJob j, int *fa
                     comb_signed(e, d);
                 }
                 const int nt = t + 1;
-                if (nt < rows) { // digit nt and its one-hot row in A
-                    if (nt == 0 && nr) {
+                if (nt < r1) { // digit nt and its one-hot row in A
+                    if (nt == r0 && nt < nr) {
                         uint32_t a[8], b[8];
                         if (live) {
                             comb_scalar(a, j, i);
@@ -374,7 +355,7 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) k_comb256(CombJob j, int *fa
 #pragma unroll
                         for (int k = 0; k < 8; ++k) dig[k * S::NT] = b[k];
                     }
-                    if (nt == nr) {
+                    if (nt == nr || (nt == r0 && nt > nr)) {
                         uint32_t b[3];
                         comb_recode_small(b, live && j.m ? j.m[i] : 0, mr);
 #pragma unroll
@@ -402,154 +383,97 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) k_comb256(CombJob j, int *fa
                     __syncwarp();
                     if ((tid & 31) == 0) mbar_arrive(&ready[wg]);
                 }
-                if (t == 0) {
+                if (t == r0) {
                     comb_first(h, e);
-                } else if (t > 0) {
+                } else if (t > r0) {
                     ge_p1p1 r;
                     ge_madd(r, h, e);
                     ge_p1p1_to_p3(h, r);
                 }
             }
-            if (live && !bad) comb_put<ACC>(CombJob::pick(j.dst, half), CombJob::pick(j.s, half), i, h);
+            if (!SPLIT && live && !bad) comb_put<ACC>(CombJob::pick(j.dst, half), CombJob::pick(j.s, half), i, h);
         }
         if (bad) *(volatile int *)fault = 1;
+    }
+    if (SPLIT) {
+        __syncwarp();
+        uint4 *x = (uint4 *)(sm + S::X) + tid; // two buffers in turn of [word][thread]
+#pragma unroll 1
+        for (unsigned to = parts / 2; to > 0; to >>= 1, x += x < (uint4 *)(sm + S::X) + 8 * S::NT ? 8 * S::NT : -8 * S::NT) {
+            if (wg < G && part >= to && part < 2 * to) {
+                const fe *const c[4] = {&h.X, &h.Y, &h.Z, &h.T};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    cluster_store(x + 2 * k * S::NT, part - to, u4_lo(*c[k]));
+                    cluster_store(x + (2 * k + 1) * S::NT, part - to, u4_hi(*c[k]));
+                }
+            }
+            cluster_sync();
+            if (wg < G && part < to) {
+                ge_p3 y;
+                ld_p3(y, x, S::NT, 0);
+                ge_addto(h, y);
+            }
+        }
+        const int half = j.h1 - 1 - (int)(tile0 / per_half);
+        const size_t i = (size_t)(tile0 % per_half) * S::NT + tid;
+        if (wg < G && part == 0 && i < j.n) comb_put<ACC>(CombJob::pick(j.dst, half), CombJob::pick(j.s, half), i, h);
     }
     tmem_sync_threads();
     if (warp == 0) tmem_free(s_taddr, S::COLS);
 }
 
-// ------------------------------------------------------------ radix 32
-
-// L lanes per unit: lane k of a unit sums its rows k, k + L, ..., then the
-// lanes' sums are added in a tree.  The table is read from L1 / L2, a row to
-// each lane (consecutive rows are consecutive words); the digits are
-// recoded by each lane.
-static constexpr int LANES_NT = 64;
-
-template <int L, bool ACC>
-__global__ void __launch_bounds__(LANES_NT) k_comb_lanes(CombJob j)
-{
-    __shared__ uint32_t s_dig[2][10][LANES_NT];
-    const size_t u = ((size_t)blockIdx.x * LANES_NT + threadIdx.x) / L;
-    const int lane = threadIdx.x % L;
-    const size_t units = j.n * (j.h1 - j.h0);
-    const bool live = u < units;
-    const int half = live ? j.h1 - 1 - (int)(u / j.n) : j.h0;
-    const size_t i = live ? u % j.n : 0;
-    const int nr = j.sc ? ENC_ROWS : 0, mr = CombJob::pick(j.mrows, half), rows = nr + mr;
-    uint32_t c[9];
-    if (nr) {
-        uint32_t a[8];
-        comb_scalar(a, j, i);
-        enc_recode(c, a, ENC_ROWS);
-#pragma unroll
-        for (int k = 0; k < 9; ++k) s_dig[0][k][threadIdx.x] = c[k];
-        s_dig[0][9][threadIdx.x] = 0u;
-    }
-    if (mr) {
-        const uint64_t m = j.m ? j.m[i] : 0;
-        const uint32_t a[8] = {(uint32_t)m, (uint32_t)(m >> 32), 0u, 0u, 0u, 0u, 0u, 0u};
-        enc_recode(c, a, mr);
-#pragma unroll
-        for (int k = 0; k < 9; ++k) s_dig[1][k][threadIdx.x] = c[k];
-        s_dig[1][9][threadIdx.x] = 0u;
-    }
-    const uint4 *tr = (const uint4 *)CombJob::pick(j.tr, half), *tm = (const uint4 *)j.tm;
-    ge_p3 h;
-    ge_p3_0(h);
-#pragma unroll 1
-    for (int t = lane; t < rows; t += L) {
-        const bool second = t >= nr;
-        const int row = second ? t - nr : t, bit = 5 * row;
-        const uint32_t lo = s_dig[second][bit >> 5][threadIdx.x], hi = s_dig[second][(bit >> 5) + 1][threadIdx.x];
-        const int d = (int)(__funnelshift_r(lo, hi, bit & 31) & 31u) - 16;
-        ge_precomp e;
-        enc_select<T32_ROWS>(e, d, (second ? tm : tr) + row);
-        if (t == lane) {
-            comb_first(h, e);
-        } else {
-            ge_p1p1 r;
-            ge_madd(r, h, e);
-            ge_p1p1_to_p3(h, r);
-        }
-    }
-    __syncwarp();
-#pragma unroll 1
-    for (int o = L / 2; o > 0; o >>= 1) {
-        ge_p3 x;
-        shfl_down_p3(x, h, o);
-        ge_addto(h, x);
-    }
-    if (live && lane == 0) comb_put<ACC>(CombJob::pick(j.dst, half), CombJob::pick(j.s, half), i, h);
-}
-
 // ------------------------------------------------------------ launchers
 
-// Up to 12 units per warp scheduler the radix-32 kernel is faster: 1,824
-// ciphertexts (6 units) 68 us, 3,648 (12) 77 us with eight lanes a unit, 108 us
-// beyond with four, against 97 us in the radix-256 kernel for any number up to
-// 128 units per SM.
-bool comb_is_wide(size_t units) { return units > (size_t)sm_count() * 48; }
-
-// Warpgroups per block: a round of 128 G units per SM takes about 90, 120 and
-// 158 us for G = 1, 2 and 3, so G = 3 for many rounds, else the one whose
-// rounds take the least (38,912 ciphertexts: 244 us with 2, 330 with 3).
-static int comb_warpgroups(size_t units)
-{
-    const size_t per_sm = (units + sm_count() - 1) / sm_count();
-    const size_t us[4] = {0, 90, 120, 158};
-    int best = 3;
-    for (int g = 2; g >= 1; --g)
-        if ((per_sm + 128 * g - 1) / (128 * g) * us[g] < (per_sm + 128 * best - 1) / (128 * best) * us[best]) best = g;
-    return best;
-}
-
-template <int G, bool ACC>
-static cudaError_t launch_256(const CombJob &j, int *fault, cudaStream_t st)
+template <int G, bool ACC, bool SPLIT>
+static cudaError_t launch_256(const CombJob &j, size_t tiles, unsigned parts, int *fault, cudaStream_t st)
 {
     using S = CombSmem<G>;
     static SmemAttr attr;
-    cudaError_t e = ensure_smem_attr(attr, (const void *)k_comb256<G, ACC>, S::BYTES);
+    cudaError_t e = ensure_smem_attr(attr, (const void *)k_comb256<G, ACC, SPLIT>, S::BYTES);
     if (e != cudaSuccess) return e;
-    const size_t tiles = (j.n + S::NT - 1) / S::NT * (j.h1 - j.h0), cap = (size_t)sm_count();
-    k_comb256<G, ACC><<<(unsigned)std::min(tiles, cap), S::NT + 128, S::BYTES, st>>>(j, fault);
-    return cudaGetLastError();
+    cudaLaunchAttribute cluster;
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = parts;
+    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((unsigned)(SPLIT ? tiles * parts : std::min<size_t>(tiles, sm_count())));
+    c.blockDim = dim3(S::NT + 128);
+    c.dynamicSmemBytes = S::BYTES;
+    c.stream = st;
+    c.attrs = &cluster;
+    c.numAttrs = SPLIT ? 1 : 0;
+    return cudaLaunchKernelEx(&c, k_comb256<G, ACC, SPLIT>, j, fault);
 }
 
-template <int L, bool ACC>
-static cudaError_t launch_lanes(const CombJob &j, cudaStream_t st)
-{
-    const size_t threads = j.n * (j.h1 - j.h0) * L;
-    k_comb_lanes<L, ACC><<<(unsigned)((threads + LANES_NT - 1) / LANES_NT), LANES_NT, 0, st>>>(j);
-    return cudaGetLastError();
-}
-
-// a job whose tables are those of tr0, tr1 (halves 0 and 1) and tm, and whose
-// m has mbits bits (0: none) in the halves of mask mhalf
+// a job whose scalars' tables are tr0 and tr1 (halves 0 and 1), m's is tm, and
+// whose m has mbits bits (0: none) in the halves of mask mhalf
 template <bool ACC>
 static cudaError_t comb_launch(CombJob j, const CombTable *tr0, const CombTable *tr1, const CombTable *tm,
                                unsigned mbits, unsigned mhalf, int *fault, cudaStream_t st)
 {
     if (j.n == 0) return cudaSuccess;
-    const size_t units = j.n * (j.h1 - j.h0);
-    const bool wide = comb_is_wide(units);
     const CombTable *tr[2] = {tr0, tr1};
     for (int h = 0; h < 2; ++h) {
-        j.tr[h] = tr[h] ? (wide ? (const void *)t256_of(*tr[h]) : (const void *)t32_of(*tr[h])) : nullptr;
-        j.mrows[h] = mbits && (mhalf >> h & 1) ? (wide ? comb_rows(mbits) : enc_digits(mbits)) : 0;
+        j.tr[h] = tr[h] ? rows_of(*tr[h]) : nullptr;
+        j.mrows[h] = mbits && (mhalf >> h & 1) ? comb_rows(mbits) : 0;
     }
-    j.tm = wide ? (const void *)t256_of(*tm) : (const void *)t32_of(*tm);
-    if (wide) {
-        switch (comb_warpgroups(units)) {
-        case 1: return launch_256<1, ACC>(j, fault, st);
-        case 2: return launch_256<2, ACC>(j, fault, st);
-        default: return launch_256<3, ACC>(j, fault, st);
-        }
+    j.tm = rows_of(*tm);
+    const size_t halves = j.h1 - j.h0, sm = sm_count();
+    auto tiles = [&](int g) { return (j.n + 128 * g - 1) / (128 * g) * halves; };
+    // Up to a tile per SM, a tile's rows are split over as many blocks as give
+    // two per SM at most.
+    const size_t t = tiles(1);
+    if (t <= sm) {
+        const unsigned parts = 8 * t <= 2 * sm ? 8 : 4 * t <= 2 * sm ? 4 : 2 * t <= 2 * sm ? 2 : 1;
+        return launch_256<1, ACC, true>(j, t, parts, fault, st);
     }
-    const size_t warps = (size_t)sm_count() * 4;
-    if (units <= 2 * warps) return launch_lanes<32, ACC>(j, st);
-    if (units <= 4 * warps) return launch_lanes<16, ACC>(j, st);
-    return launch_lanes<8, ACC>(j, st);
+    // Beyond, a round of a tile of 256 units per SM takes about 120 us, of 384
+    // about 158: 384 for many rounds, else what takes the least (38,912
+    // ciphertexts: 244 us at 256, 330 at 384; 1,048,576: 6.09 and 5.54 ms).
+    const size_t r2 = (tiles(2) + sm - 1) / sm, r3 = (tiles(3) + sm - 1) / sm;
+    if (r2 * 120 < r3 * 158) return launch_256<2, ACC, false>(j, tiles(2), 1, fault, st);
+    return launch_256<3, ACC, false>(j, tiles(3), 1, fault, st);
 }
 
 template <bool ACC>

@@ -102,6 +102,36 @@ FT_DEV_TM void umma_commit(uint64_t *b)
                  : "memory");
 }
 
+// thread-block clusters: this block's rank and their number, a barrier of all
+// threads of the cluster, and a store into the same place of another block's
+// shared memory
+FT_DEV_TM unsigned cluster_rank()
+{
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+
+FT_DEV_TM unsigned cluster_size()
+{
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+
+FT_DEV_TM void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+FT_DEV_TM void cluster_store(uint4 *local, unsigned rank, uint4 v)
+{
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(local)), "r"(rank));
+    asm volatile("st.shared::cluster.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+                 : "memory");
+}
+
 FT_DEV_TM void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 
 FT_DEV_TM void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
