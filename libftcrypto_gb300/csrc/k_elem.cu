@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(256) k_broadcast(uint4 *p, size_t s, size_t n,
 
 __global__ void __launch_bounds__(128, 4) k_add(uint4 *r, size_t rs, const uint4 *a, size_t as, size_t n, int sub)
 {
+    after_previous();
     FT_GRID_LOOP(i, n)
     {
         ge_p3 x, y;
@@ -82,6 +83,7 @@ __global__ void __launch_bounds__(128, 4) k_add(uint4 *r, size_t rs, const uint4
 __global__ void __launch_bounds__(128, 4) k_add_ct(uint4 *r1, size_t r1s, const uint4 *a1, size_t a1s, uint4 *r2,
                                                    size_t r2s, const uint4 *a2, size_t a2s, size_t n, int sub)
 {
+    after_previous();
     FT_GRID_LOOP(j, 2 * n)
     {
         const bool hi = j >= n;
@@ -588,10 +590,19 @@ cudaError_t or_words(uint64_t *acc, const uint64_t *v, size_t n, cudaStream_t st
     FT_LAUNCH(k_or_words, n, 256, (unsigned long long *)acc, v, n);
 }
 cudaError_t broadcast(View d, size_t n, View q, cudaStream_t st) { FT_LAUNCH(k_broadcast, n, 256, d.p, d.s, n, q.p, q.s); }
-cudaError_t add(View r, View a, size_t n, int sub, cudaStream_t st) { FT_LAUNCH(k_add, n, 128, r.p, r.s, a.p, a.s, n, sub); }
+// (a block for every 128 points: 1,048,576 ciphertexts in 165 us, 178 with the
+// 1,216 blocks of the other kernels)
+static unsigned blocks_for(size_t n) { return (unsigned)((n + 127) / 128 < 0x7fffffff ? (n + 127) / 128 : 0x7fffffff); }
+
+cudaError_t add(View r, View a, size_t n, int sub, cudaStream_t st)
+{
+    if (n == 0) return cudaSuccess;
+    return launch_next(k_add, blocks_for(n), 128, 0, st, r.p, r.s, a.p, a.s, n, sub);
+}
 cudaError_t add_ct(View r1, View r2, View a1, View a2, size_t n, int sub, cudaStream_t st)
 {
-    FT_LAUNCH(k_add_ct, 2 * n, 128, r1.p, r1.s, a1.p, a1.s, r2.p, r2.s, a2.p, a2.s, n, sub);
+    if (n == 0) return cudaSuccess;
+    return launch_next(k_add_ct, blocks_for(2 * n), 128, 0, st, r1.p, r1.s, a1.p, a1.s, r2.p, r2.s, a2.p, a2.s, n, sub);
 }
 cudaError_t neg(View v, size_t n, cudaStream_t st) { FT_LAUNCH(k_neg, n, 256, v.p, v.s, n); }
 cudaError_t index_nonzero(int64_t *o, View v, size_t n, cudaStream_t st) { FT_LAUNCH(k_index, n, 256, o, v.p, v.s, n); }

@@ -109,6 +109,15 @@ FT_DEV void points_wait()
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// First statement of a kernel launched by launch_next (internal.h): the next
+// such launch of the stream may place its blocks from here on, and nothing
+// of the launches before is read or overwritten before they are done.
+FT_DEV void after_previous()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // grid-stride loop bounds in size_t
 #define FT_GRID_LOOP(i, n) \
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += (size_t)blockDim.x * gridDim.x)
