@@ -17,7 +17,7 @@
 // A table row is a K-major B operand of COMB_K = 128 entries x COMB_N = 80
 // columns (72 used): element (column n, entry k) at (k / 8) * 16 COMB_N +
 // n * 16 + (k % 8) * 2, entry k = (k + 1) * 256^row * Q.  Column 24 f + 8 c + w
-// is part c of word w of coordinate f (y+x, y-x, 2dxy).
+// is part c of word w of coordinate f ((y+x)/2, (y-x)/2, dxy).
 #pragma once
 #include "ge.cuh"
 
@@ -68,22 +68,20 @@ FT_DEV int comb_offset(int n, int k) { return (k >> 3) * COMB_CHUNK + n * 16 + (
 // part c of a table word
 FT_DEV uint32_t comb_part(uint32_t w, int c) { return c == 0 ? w & 2047u : c == 1 ? w >> 11 & 2047u : w >> 22; }
 
-// the table word of its three parts as f32 integers: 2^23 + p0 + 2048 p1 has
-// the low 22 bits in place; 2^23 + 724 + p2 shifted by 22 adds the high ten
-// and (724 = 0x2d4) cancels the exponent bits of the first
-FT_DEV uint32_t comb_word(float p0, float p1, float p2)
+// The product adds 2^23 to every column, so that its f32 is the integer with
+// the exponent bits 0x4b000000, and 724 to the columns of part 2: 16 entries
+// more, the same in all rows, of which every row of A selects the first 2048
+// times and the second once (the f16 pair COMB_MAGIC_A).  The pair of column n:
+static constexpr uint32_t COMB_MAGIC_A = 0x3c006800u;
+
+FT_DEV uint32_t comb_magic(int n)
 {
-    const float lo = p1 * 2048.0f + (p0 + 8388608.0f), hi = p2 + 8389332.0f;
-    uint32_t a, b;
-#ifdef FT_HOST_EMULATION
-    memcpy(&a, &lo, 4);
-    memcpy(&b, &hi, 4);
-#else
-    a = __float_as_uint(lo);
-    b = __float_as_uint(hi);
-#endif
-    return (b << 22) + a;
+    return n >= 72 ? 0u : (n / 8 % 3 == 2 ? 0x61a80000u : 0u) | 0x6c00u; // 4096 and 724 or 0
 }
+
+// the table word of its three columns' bits: shifted by 11 and 22 the exponent
+// bits are gone, and 724 << 22 (0x2d4 << 22) cancels those of the first
+FT_DEV uint32_t comb_word(uint32_t p0, uint32_t p1, uint32_t p2) { return (p2 << 22) + (p1 << 11) + p0; }
 
 // -f for the canonical f under the mask (a table word group: f < 2^255)
 FT_DEV void comb_neg(fe &f, uint32_t m)
@@ -97,12 +95,10 @@ FT_DEV void comb_neg(fe &f, uint32_t m)
     for (int k = 0; k < 8; ++k) f.v[k] = r[k];
 }
 
-// the entry of |d| negated for d < 0 (the mask neg), (1, 1, 0) for d = 0
+// the entry of |d| negated for d < 0
 FT_DEV void comb_signed(ge_precomp &t, int d)
 {
-    const uint32_t id = d == 0 ? 1u : 0u, neg = 0u - ((uint32_t)d >> 31);
-    t.yplusx.v[0] |= id;
-    t.yminusx.v[0] |= id;
+    const uint32_t neg = 0u - ((uint32_t)d >> 31);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
         const uint32_t p = t.yplusx.v[k], q = t.yminusx.v[k];
@@ -112,16 +108,84 @@ FT_DEV void comb_signed(ge_precomp &t, int d)
     comb_neg(t.xy2d, neg);
 }
 
-// h = the entry itself: with 2x = (y+x) - (y-x) and 2y the sum, (4x : 4y : 4 :
-// 4xy), one multiplication instead of the seven of an addition to 0
+// ---- additions of halved entries on coordinates below 2^255 + 1463
+//
+// With (y+x)/2, (y-x)/2 and dxy in an entry the four intermediate coordinates
+// come out halved, the same point, and 2 Z is Z.  The products are folded at
+// bit 255 instead of 256, to below 2^255 + 19 * 77, so that a sum of two is
+// below 2^256 + 2926 and its carry is repaid in the lowest word: 10 instructions
+// instead of 19, and one sum fewer (1,048,576 ciphertexts 5.45 -> 5.22 ms).
+
+FT_DEV void fold_tight(fe &h, const uint32_t t[16])
+{
+    uint32_t r[8], r8;
+    fold_288(r, r8, t);
+    const uint32_t top = r8 << 1 | r[7] >> 31; // at most 77
+    r[7] &= 0x7fffffffu;
+    h.v[0] = mad_lo_cc(top, 19u, r[0]);
+#pragma unroll
+    for (int k = 1; k < 7; ++k) h.v[k] = addc_cc(r[k], 0u);
+    h.v[7] = addc(r[7], 0u);
+}
+
+FT_DEV void mul_tight(fe &h, const fe &a, const fe &b)
+{
+    uint32_t t[16];
+    mul_wide(t, a, b);
+    fold_tight(h, t);
+}
+
+FT_DEV void mul_tight_x2(fe &h1, const fe &a1, const fe &b1, fe &h2, const fe &a2, const fe &b2)
+{
+    uint32_t t1[16], t2[16];
+    mul_wide2(t1, a1, b1, t2, a2, b2);
+    fold_tight(h1, t1);
+    fold_tight(h2, t2);
+}
+
+// a + b of two such coordinates, below 2^256
+FT_DEV void add_tight(fe &h, const fe &a, const fe &b)
+{
+    uint32_t r[8];
+    r[0] = add_cc(a.v[0], b.v[0]);
+#pragma unroll
+    for (int k = 1; k < 8; ++k) r[k] = addc_cc(a.v[k], b.v[k]);
+    const uint32_t c = addc(0u, 0u);
+    r[0] += 38u * c; // r < 2926 where c is 1
+#pragma unroll
+    for (int k = 0; k < 8; ++k) h.v[k] = r[k];
+}
+
+// h += the entry t (ge_madd and ge_p1p1_to_p3 on halves)
+FT_DEV void comb_add(ge_p3 &h, const ge_precomp &t)
+{
+    fe e, f, g, k;
+    add_tight(g, h.Y, h.X);
+    fe_sub(f, h.Y, h.X);
+    mul_tight_x2(g, g, t.yplusx, f, f, t.yminusx);
+    fe_sub(e, g, f);
+    add_tight(k, g, f);
+    mul_tight(g, t.xy2d, h.T);
+    fe_sub(f, h.Z, g);
+    add_tight(g, h.Z, g);
+    mul_tight_x2(h.X, e, f, h.Y, k, g);
+    mul_tight_x2(h.Z, g, f, h.T, e, k);
+}
+
+// h = the entry itself: x = (y+x)/2 - (y-x)/2, y their sum (both below 2^255)
 FT_DEV void comb_first(ge_p3 &h, const ge_precomp &t)
 {
-    fe x2, y2;
-    fe_sub(x2, t.yplusx, t.yminusx);
-    fe_add(y2, t.yplusx, t.yminusx);
-    fe_mul(h.T, x2, y2);
-    fe_add(h.X, x2, x2);
-    fe_add(h.Y, y2, y2);
-    fe_0(h.Z);
-    h.Z.v[0] = 4;
+    fe one;
+    fe_1(one);
+    fe_sub(h.X, t.yplusx, t.yminusx);
+    fe_add(h.Y, t.yplusx, t.yminusx);
+    mul_tight(h.T, h.X, h.Y);
+    mul_tight_x2(h.X, h.X, one, h.Y, h.Y, one); // below 2^255 + 1463
+    h.Z = one;
 }
+
+// 1/2 mod p = 2^254 - 9
+FT_DEV fe fe_half() { return fe_const(0xfffffff7u, ~0u, ~0u, ~0u, ~0u, ~0u, ~0u, 0x3fffffffu); }
+
+// word w of the identity's entry (1/2, 1/2, 0)
+FT_DEV uint32_t comb_identity(int w) { return w >= 16 ? 0u : (w & 7) == 0 ? 0xfffffff7u : (w & 7) == 7 ? 0x3fffffffu : ~0u; }

@@ -100,9 +100,9 @@ FT_DEV void fe_neg(fe &h, const fe &f)
 // ms for the constant-time ladder of 1,048,576 points, same words.
 // (Forming 38 t_hi as (t_hi << 5) + (t_hi << 2) + (t_hi << 1) with funnel
 // shifts and carry chains instead measured slower: 23.7 ms.)
-FT_DEV void fe_fold512(fe &h, const uint32_t t[16])
+FT_DEV void fold_288(uint32_t r[8], uint32_t &r8, const uint32_t t[16])
 {
-    uint32_t r[8], r8, o[8];
+    uint32_t o[8];
     r[0] = mad_lo_cc(t[8], 38u, t[0]);
     r[1] = madc_hi_cc(t[8], 38u, t[1]);
 #pragma unroll
@@ -120,6 +120,12 @@ FT_DEV void fe_fold512(fe &h, const uint32_t t[16])
 #pragma unroll
     for (int k = 2; k < 8; ++k) r[k] = addc_cc(r[k], o[k - 1]);
     r8 = addc(r8, o[7]);
+}
+
+FT_DEV void fe_fold512(fe &h, const uint32_t t[16])
+{
+    uint32_t r[8], r8;
+    fold_288(r, r8, t);
     // value = r + r8 * 2^256 with r8 <= 38
     r[0] = mad_lo_cc(r8, 38u, r[0]);
 #pragma unroll

@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(32) k_comb_bases(uint4 *out, const uint4 *q, s
     }
 }
 
-// k * P as an affine table entry, k < 2^bits public
+// k * P as a halved affine entry (comb256.cuh), k < 2^bits public
 FT_DEV void comb_entry(ge_precomp &t, const uint4 *base, int k, int bits)
 {
     ge_p3 P, acc;
@@ -81,14 +81,16 @@ FT_DEV void comb_entry(ge_precomp &t, const uint4 *base, int k, int bits)
             ge_p1p1_to_p3(acc, r);
         }
     }
-    fe zi, x, y;
+    fe zi, x, y, xy;
     fe_inv(zi, acc.Z);
     fe_mul(x, acc.X, zi);
     fe_mul(y, acc.Y, zi);
+    fe_mul(xy, x, y);
+    fe_mul(t.xy2d, xy, fe_d());
+    fe_mul(x, x, fe_half());
+    fe_mul(y, y, fe_half());
     fe_add(t.yplusx, y, x);
     fe_sub(t.yminusx, y, x);
-    fe_mul(x, x, y);
-    fe_mul(t.xy2d, x, fe_d2());
     fe_canon(t.yplusx, t.yplusx);
     fe_canon(t.yminusx, t.yminusx);
     fe_canon(t.xy2d, t.xy2d);
@@ -175,15 +177,17 @@ static constexpr uint32_t COMB_IDESC = umma_idesc_f16(128, COMB_N);
 
 // A block of G warpgroups: three table rows and the recoded scalars in shared
 // memory; in tensor memory, per warpgroup, its products (COMB_N columns) and
-// its one-hot rows (COMB_K / 2 columns).  Shared memory is padded so that no
-// block's tensor-memory allocation waits for another's: one block per SM, or
-// two of G = 1, which take half the columns each.
+// its one-hot rows (COMB_K / 2 columns, then 8 for the 16 constant entries).
+// Shared memory is padded so that no block's tensor-memory allocation waits for
+// another's: one block per SM, or two of G = 1, which take half the columns
+// each.
 template <int G>
 struct CombSmem {
     static constexpr int NT = 128 * G;
-    static constexpr uint32_t A = COMB_N, PER_WG = COMB_N + COMB_K / 2, COLS = G == 1 ? 256 : 512;
+    static constexpr uint32_t A = COMB_N, PER_WG = COMB_N + COMB_K / 2 + 8, COLS = G == 1 ? 256 : 512;
     static_assert(G * PER_WG <= COLS, "tensor memory");
-    static constexpr size_t B = 0, DIG = 3 * (size_t)COMB_ROW_BYTES, X = DIG + (size_t)8 * NT * 4;
+    static constexpr size_t B = 0, MAGIC = 3 * (size_t)COMB_ROW_BYTES,
+                            DIG = MAGIC + 2 * COMB_CHUNK, X = DIG + (size_t)8 * NT * 4;
     static constexpr size_t USED = X + (G == 1 ? 2 * (size_t)8 * NT * 16 : 0); // X: points from the cluster's others
     static constexpr size_t BYTES = std::max(USED, (size_t)(G == 1 ? 80 : 116) * 1024);
 };
@@ -202,7 +206,11 @@ struct CombSmem {
 // step and one of its threads issuing; 6.25 to 6.50 with the last warp of a
 // warpgroup to be ready issuing (it takes that warp 1,100 cycles, in which its
 // own row and so its warpgroup's next product wait); 5.55 with one warp
-// issuing for all, on whose scheduler the computing warps fell behind.
+// issuing for all, on whose scheduler the computing warps fell behind; 5.53
+// with four; 5.45 with the 2^23 that makes integers of the f32 in the product;
+// 5.22 with comb_add.  (What is added to the multiplications is not hidden by
+// them: about a cycle an instruction.  The one-hot rows written by the issuing
+// warps instead: 5.69 against 5.45.)
 // SPLIT (G = 1): the blocks of a cluster (1, 2, 4 or 8) take a part of a tile's
 // rows each, then add their points up in pairs, through the shared memory of
 // the lower block of each pair.
@@ -238,6 +246,13 @@ __global__ void __launch_bounds__(128 * (G + 1), SPLIT ? 2 : 1) k_comb256(CombJo
         }
         mbar_fence_init();
     }
+    if (tid < COMB_N) { // the 16 entries after the row's, the same for every row
+        uint4 *m = (uint4 *)(sm + S::MAGIC) + tid;
+        const uint32_t id = tid < 72 ? comb_part(comb_identity(tid / 24 * 8 + (tid & 7)), tid / 8 % 3) : 0u;
+        m[0] = make_uint4(comb_magic(tid), __half_as_ushort(__uint2half_rn(id)), 0u, 0u);
+        m[COMB_N] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    fence_async_smem();
     tmem_sync_threads();
     if (SPLIT) cluster_sync(); // every block of it runs
 
@@ -295,9 +310,11 @@ __global__ void __launch_bounds__(128 * (G + 1), SPLIT ? 2 : 1) k_comb256(CombJo
                 }
                 tmem_fence_after();
                 const uint64_t bd = umma_desc(smem_addr(sm + S::B + buf * COMB_ROW_BYTES), COMB_CHUNK, 128);
+                umma_f16_ta(dt, dt + S::A + COMB_K / 2, umma_desc(smem_addr(sm + S::MAGIC), COMB_CHUNK, 128), COMB_IDESC,
+                            false);
 #pragma unroll
                 for (int k = 0; k < COMB_K / 16; ++k)
-                    umma_f16_ta(dt, dt + S::A + 8u * k, bd + k * (2 * COMB_CHUNK >> 4), COMB_IDESC, k != 0);
+                    umma_f16_ta(dt, dt + S::A + 8u * k, bd + k * (2 * COMB_CHUNK >> 4), COMB_IDESC, true);
                 umma_commit(&done[g]);
                 umma_commit(&empty[buf]);
                 if (++buf == 3) {
@@ -310,6 +327,10 @@ __global__ void __launch_bounds__(128 * (G + 1), SPLIT ? 2 : 1) k_comb256(CombJo
     } else {
         uint32_t *dig = (uint32_t *)(sm + S::DIG) + tid;
         const uint32_t my_tmem = tmem_warp_addr(s_taddr + S::PER_WG * wg, warp, 0u);
+        {
+            const uint32_t w[8] = {COMB_MAGIC_A, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+            tmem_st8(my_tmem + S::A + COMB_K / 2, w); // what the rows multiply those entries by
+        }
         unsigned q = 0; // steps so far
         bool bad = false;
 #pragma unroll 1
@@ -333,7 +354,7 @@ __global__ void __launch_bounds__(128 * (G + 1), SPLIT ? 2 : 1) k_comb256(CombJo
                     fe *const f[3] = {&e.yplusx, &e.yminusx, &e.xy2d};
 #pragma unroll
                     for (int g = 0; g < 3; ++g) {
-                        float p[24];
+                        uint32_t p[24];
                         tmem_ld24(my_tmem + 24 * g, p);
 #pragma unroll
                         for (int k = 0; k < 8; ++k) f[g]->v[k] = comb_word(p[k], p[8 + k], p[16 + k]);
@@ -378,6 +399,9 @@ __global__ void __launch_bounds__(128 * (G + 1), SPLIT ? 2 : 1) k_comb256(CombJo
                         }
                         tmem_st8(my_tmem + S::A + c, w);
                     }
+                    const uint32_t zh = 0x63ffu; // 1023.5, x for the digit 0; 0 in the high half, which x is not
+                    const __half2 zero = __heq2(x, *(const __half2 *)&zh);
+                    tmem_st1(my_tmem + S::A + COMB_K / 2 + 1, *(const uint32_t *)&zero);
                     tmem_wait_st();
                     tmem_fence_before();
                     __syncwarp();
@@ -386,9 +410,7 @@ __global__ void __launch_bounds__(128 * (G + 1), SPLIT ? 2 : 1) k_comb256(CombJo
                 if (t == r0) {
                     comb_first(h, e);
                 } else if (t > r0) {
-                    ge_p1p1 r;
-                    ge_madd(r, h, e);
-                    ge_p1p1_to_p3(h, r);
+                    comb_add(h, e);
                 }
             }
             if (!SPLIT && live && !bad) comb_put<ACC>(CombJob::pick(j.dst, half), CombJob::pick(j.s, half), i, h);

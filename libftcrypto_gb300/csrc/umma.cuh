@@ -69,6 +69,9 @@ FT_DEV_TM void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *b
                  : "memory");
 }
 
+// generic-proxy writes of shared memory made visible to the tensor core
+FT_DEV_TM void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
 // shared-memory matrix descriptor: K-major, no swizzle; `lbo` bytes between
 // core matrices along K, `sbo` along the rows
 FT_DEV_TM uint64_t umma_desc(uint32_t addr, uint32_t lbo, uint32_t sbo)
@@ -136,17 +139,22 @@ FT_DEV_TM void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_
 
 FT_DEV_TM void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+FT_DEV_TM void tmem_st1(uint32_t ta, uint32_t v)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(ta), "r"(v) : "memory");
+}
+
 // 24 consecutive columns of the thread's lane
-FT_DEV_TM void tmem_ld24(uint32_t ta, float r[24])
+FT_DEV_TM void tmem_ld24(uint32_t ta, uint32_t r[24])
 {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%24];\n\t"
                  "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23}, "
                  "[%25];\n\t"
                  "tcgen05.wait::ld.sync.aligned;"
-                 : "=&f"(r[0]), "=&f"(r[1]), "=&f"(r[2]), "=&f"(r[3]), "=&f"(r[4]), "=&f"(r[5]), "=&f"(r[6]),
-                   "=&f"(r[7]), "=&f"(r[8]), "=&f"(r[9]), "=&f"(r[10]), "=&f"(r[11]), "=&f"(r[12]), "=&f"(r[13]),
-                   "=&f"(r[14]), "=&f"(r[15]), "=&f"(r[16]), "=&f"(r[17]), "=&f"(r[18]), "=&f"(r[19]), "=&f"(r[20]),
-                   "=&f"(r[21]), "=&f"(r[22]), "=&f"(r[23])
+                 : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]),
+                   "=&r"(r[7]), "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]), "=&r"(r[12]), "=&r"(r[13]),
+                   "=&r"(r[14]), "=&r"(r[15]), "=&r"(r[16]), "=&r"(r[17]), "=&r"(r[18]), "=&r"(r[19]), "=&r"(r[20]),
+                   "=&r"(r[21]), "=&r"(r[22]), "=&r"(r[23])
                  : "r"(ta), "r"(ta + 8u)
                  : "memory");
 }

@@ -10,6 +10,16 @@
 #include "../../libftcrypto_gb300/csrc/fe_inv.cuh"
 
 static std::vector<float> g_tab; // [row][offset / 2]
+static bool g_tight = true;
+
+// f < 2^255 + 1463
+static bool tight(const fe &f)
+{
+    if (!(f.v[7] >> 31)) return true;
+    for (int k = 1; k < 8; ++k)
+        if (f.v[k] != (k == 7 ? 0x80000000u : 0u)) return false;
+    return f.v[0] < 1463u;
+}
 
 static void put_row(int row, const ge_p3 &base)
 {
@@ -18,14 +28,16 @@ static void put_row(int row, const ge_p3 &base)
     ge_p3_to_cached(c, base);
     float *o = &g_tab[(size_t)row * COMB_ROW_BYTES / 2];
     for (int k = 0; k < COMB_K; ++k) {
-        fe zi, x, y, e[3];
+        fe zi, x, y, xy, e[3];
         fe_inv(zi, acc.Z);
         fe_mul(x, acc.X, zi);
         fe_mul(y, acc.Y, zi);
+        fe_mul(xy, x, y);
+        fe_mul(e[2], xy, fe_d());
+        fe_mul(x, x, fe_half());
+        fe_mul(y, y, fe_half());
         fe_add(e[0], y, x);
         fe_sub(e[1], y, x);
-        fe_mul(x, x, y);
-        fe_mul(e[2], x, fe_d2());
         for (int j = 0; j < 3; ++j) {
             fe_canon(e[j], e[j]);
             for (int w = 0; w < 8; ++w)
@@ -37,6 +49,13 @@ static void put_row(int row, const ge_p3 &base)
     }
 }
 
+// the value of a normal f16, 0 for 0
+static float half(uint32_t bits)
+{
+    bits &= 0xffffu;
+    return bits ? (float)((bits & 1023u) + 1024u) * (float)(1u << (bits >> 10)) / 33554432.0f : 0.0f;
+}
+
 static void add_row(ge_p3 &h, bool first, int row, int d)
 {
     ge_precomp e;
@@ -44,21 +63,43 @@ static void add_row(ge_p3 &h, bool first, int row, int d)
     fe *f[3] = {&e.yplusx, &e.yminusx, &e.xy2d};
     const float *o = &g_tab[(size_t)row * COMB_ROW_BYTES / 2];
     for (int w = 0; w < 24; ++w) {
-        float p[3];
-        for (int c = 0; c < 3; ++c) p[c] = k < 0 ? 0.0f : o[comb_offset(24 * (w / 8) + 8 * c + w % 8, k) / 2];
+        uint32_t p[3];
+        for (int c = 0; c < 3; ++c) {
+            const int n = 24 * (w / 8) + 8 * c + w % 8;
+            const uint32_t m = comb_magic(n);
+            const float x = half(COMB_MAGIC_A) * half(m) + half(COMB_MAGIC_A >> 16) * half(m >> 16) +
+                            (k < 0 ? (float)comb_part(comb_identity(w), c) : o[comb_offset(n, k) / 2]);
+            memcpy(&p[c], &x, 4);
+        }
         f[w / 8]->v[w % 8] = comb_word(p[0], p[1], p[2]);
     }
     comb_signed(e, d);
     if (first) {
         comb_first(h, e);
     } else {
-        ge_p1p1 r;
-        ge_madd(r, h, e);
-        ge_p1p1_to_p3(h, r);
+        comb_add(h, e);
+        for (const fe *c : {&h.X, &h.Y, &h.Z, &h.T}) g_tight = g_tight && tight(*c);
     }
 }
 
 extern "C" {
+
+// whether every coordinate so far was below 2^255 + 1463
+int hc_comb256_tight(void) { return g_tight; }
+
+// mul_tight's bound on any operands, add_tight's on the largest it may see
+int hc_comb256_field(const uint8_t *a32, const uint8_t *b32, uint8_t *prod32, uint8_t *sum32)
+{
+    fe a, b, p, s;
+    memcpy(a.v, a32, 32);
+    memcpy(b.v, b32, 32);
+    mul_tight(p, a, b);
+    memcpy(prod32, p.v, 32);
+    add_tight(s, p, p);
+    memcpy(sum32, s.v, 32);
+    return tight(p);
+}
+
 
 void hc_comb256_table(const uint8_t *q128)
 {

@@ -1,8 +1,10 @@
 """The radix-256 comb (csrc/comb256.cuh), compiled for the host: digits, table
-words split into f16 integers and put together again, signed entries and the
-first row's point, against the oracle's products."""
+words split into f16 integers and put together again, signed entries, the first
+row's point and the additions, against the oracle's products, and the bound
+that the additions' coordinates keep."""
 import ctypes
 import os
+import random
 import subprocess
 
 import numpy as np
@@ -40,6 +42,22 @@ def test_products(hc, orc):
     assert dig[:, :31].min() >= -128 and dig[:, :31].max() <= 127 and dig[:, 31].min() >= 0 and dig[:, 31].max() <= 128
     assert (dig[:, 31] == 128).any()
     assert (orc.encode(pts) == orc.encode(orc.from_scalars(sc))).all()
+    assert hc.hc_comb256_tight() == 1
+
+
+def test_tight_field(hc):
+    P = 2**255 - 19
+    rnd = random.Random(3)
+    edge = [0, 1, 19, P - 1, P, P + 1, 2**255 - 1, 2**255, 2**255 + 1462, 2**256 - 1, 2**256 - 38, 2**256 - 39]
+    # operands whose product is just below and above 2^255 (mod p)
+    vals = edge + [rnd.getrandbits(256) for _ in range(2000)]
+    pairs = [(a, b) for a in edge for b in edge] + [(vals[i], vals[(7 * i + 5) % len(vals)]) for i in range(len(vals))]
+    pairs += [(x, pow(x, -1, P) * t % P) for x in vals[12:200] for t in (P - 1, P - 2, P - 1462, 1, 2, 1443, 1444)]
+    buf = [ctypes.create_string_buffer(32) for _ in range(2)]
+    for a, b in pairs:
+        assert hc.hc_comb256_field(a.to_bytes(32, "little"), b.to_bytes(32, "little"), buf[0], buf[1]) == 1
+        prod, total = (int.from_bytes(x.raw, "little") for x in buf)
+        assert prod % P == a * b % P and total % P == 2 * a * b % P
 
 
 @pytest.mark.parametrize("bits", [1, 7, 8, 15, 16, 31, 32, 63, 64])
