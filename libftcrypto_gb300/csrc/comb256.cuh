@@ -108,65 +108,23 @@ FT_DEV void comb_signed(ge_precomp &t, int d)
     comb_neg(t.xy2d, neg);
 }
 
-// ---- additions of halved entries on coordinates below 2^255 + 1463
+// ---- additions of halved entries, on tight coordinates (fe.cuh)
 //
 // With (y+x)/2, (y-x)/2 and dxy in an entry the four intermediate coordinates
-// come out halved, the same point, and 2 Z is Z.  The products are folded at
-// bit 255 instead of 256, to below 2^255 + 19 * 77, so that a sum of two is
-// below 2^256 + 2926 and its carry is repaid in the lowest word: 10 instructions
-// instead of 19, and one sum fewer (1,048,576 ciphertexts 5.45 -> 5.22 ms).
-
-FT_DEV void fold_tight(fe &h, const uint32_t t[16])
-{
-    uint32_t r[8], r8;
-    fold_288(r, r8, t);
-    const uint32_t top = r8 << 1 | r[7] >> 31; // at most 77
-    r[7] &= 0x7fffffffu;
-    h.v[0] = mad_lo_cc(top, 19u, r[0]);
-#pragma unroll
-    for (int k = 1; k < 7; ++k) h.v[k] = addc_cc(r[k], 0u);
-    h.v[7] = addc(r[7], 0u);
-}
-
-FT_DEV void mul_tight(fe &h, const fe &a, const fe &b)
-{
-    uint32_t t[16];
-    mul_wide(t, a, b);
-    fold_tight(h, t);
-}
-
-FT_DEV void mul_tight_x2(fe &h1, const fe &a1, const fe &b1, fe &h2, const fe &a2, const fe &b2)
-{
-    uint32_t t1[16], t2[16];
-    mul_wide2(t1, a1, b1, t2, a2, b2);
-    fold_tight(h1, t1);
-    fold_tight(h2, t2);
-}
-
-// a + b of two such coordinates, below 2^256
-FT_DEV void add_tight(fe &h, const fe &a, const fe &b)
-{
-    uint32_t r[8];
-    r[0] = add_cc(a.v[0], b.v[0]);
-#pragma unroll
-    for (int k = 1; k < 8; ++k) r[k] = addc_cc(a.v[k], b.v[k]);
-    const uint32_t c = addc(0u, 0u);
-    r[0] += 38u * c; // r < 2926 where c is 1
-#pragma unroll
-    for (int k = 0; k < 8; ++k) h.v[k] = r[k];
-}
+// come out halved, the same point, and 2 Z is Z: one sum fewer, and the others
+// tight (1,048,576 ciphertexts 5.45 -> 5.22 ms).
 
 // h += the entry t (ge_madd and ge_p1p1_to_p3 on halves)
 FT_DEV void comb_add(ge_p3 &h, const ge_precomp &t)
 {
     fe e, f, g, k;
     add_tight(g, h.Y, h.X);
-    fe_sub(f, h.Y, h.X);
+    sub_tight(f, h.Y, h.X);
     mul_tight_x2(g, g, t.yplusx, f, f, t.yminusx);
-    fe_sub(e, g, f);
+    sub_tight(e, g, f);
     add_tight(k, g, f);
     mul_tight(g, t.xy2d, h.T);
-    fe_sub(f, h.Z, g);
+    sub_tight(f, h.Z, g);
     add_tight(g, h.Z, g);
     mul_tight_x2(h.X, e, f, h.Y, k, g);
     mul_tight_x2(h.Z, g, f, h.T, e, k);
@@ -180,7 +138,7 @@ FT_DEV void comb_first(ge_p3 &h, const ge_precomp &t)
     fe_sub(h.X, t.yplusx, t.yminusx);
     fe_add(h.Y, t.yplusx, t.yminusx);
     mul_tight(h.T, h.X, h.Y);
-    mul_tight_x2(h.X, h.X, one, h.Y, h.Y, one); // below 2^255 + 1463
+    mul_tight_x2(h.X, h.X, one, h.Y, h.Y, one);
     h.Z = one;
 }
 

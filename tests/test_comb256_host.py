@@ -53,11 +53,11 @@ def test_tight_field(hc):
     vals = edge + [rnd.getrandbits(256) for _ in range(2000)]
     pairs = [(a, b) for a in edge for b in edge] + [(vals[i], vals[(7 * i + 5) % len(vals)]) for i in range(len(vals))]
     pairs += [(x, pow(x, -1, P) * t % P) for x in vals[12:200] for t in (P - 1, P - 2, P - 1462, 1, 2, 1443, 1444)]
-    buf = [ctypes.create_string_buffer(32) for _ in range(2)]
+    buf = [ctypes.create_string_buffer(32) for _ in range(3)]
     for a, b in pairs:
-        assert hc.hc_comb256_field(a.to_bytes(32, "little"), b.to_bytes(32, "little"), buf[0], buf[1]) == 1
-        prod, total = (int.from_bytes(x.raw, "little") for x in buf)
-        assert prod % P == a * b % P and total % P == 2 * a * b % P
+        assert hc.hc_comb256_field(a.to_bytes(32, "little"), b.to_bytes(32, "little"), *buf) == 1
+        prod, total, diff = (int.from_bytes(x.raw, "little") for x in buf)
+        assert prod % P == a * b % P and total % P == 2 * a * b % P and diff % P == (a - b) % P
 
 
 @pytest.mark.parametrize("bits", [1, 7, 8, 15, 16, 31, 32, 63, 64])
