@@ -141,9 +141,22 @@ bool host_is_pinned(const void *p)
     return at.type == cudaMemoryTypeHost;
 }
 
-// (Kernels writing exports straight into pinned caller memory over the
-// host link measured 10x slower than the conversion into device memory
-// followed by one copy: 13.1 against 1.24 ms for 1,048,576 raw points.)
+// Where a kernel may write the caller's `bytes` bytes itself: pinned memory as
+// the device addresses it, 16-byte aligned; else nullptr.
+uint8_t *device_view_of_host(uint8_t *p, size_t bytes)
+{
+    cudaPointerAttributes at, end;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess ||
+        cudaPointerGetAttributes(&end, p + bytes - 1) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    uint8_t *d = (uint8_t *)at.devicePointer;
+    if (at.type != cudaMemoryTypeHost || end.type != cudaMemoryTypeHost || !d || (uintptr_t)d % 16 ||
+        (uint8_t *)end.devicePointer != d + bytes - 1)
+        return nullptr;
+    return d;
+}
 
 // copy from caller memory: the caller may reuse `src` when this returns
 cudaError_t h2d(void *dst, const void *src, size_t bytes)
@@ -209,6 +222,12 @@ bool quiet_since_mark(const_ft_ge25519_array a)
     return a->ready && !a->exposed.load() && a->touch.load() == a->ready_touch;
 }
 
+// whether its writer marked a first part too (mark_part)
+bool has_parts(const_ft_ge25519_array a)
+{
+    return quiet_since_mark(a) && a->part && a->part_end > 0 && a->part_end < a->n;
+}
+
 // The stream and the device buffer (at least `bytes`) an export of a
 // converts and copies on.  When the call that last wrote a marked it and
 // nothing has used a since, that is the transfer stream after a wait for
@@ -236,7 +255,7 @@ cudaError_t export_begin(const_ft_ge25519_array a, size_t bytes, void **buf, cud
         if ((e = cudaMallocFromPoolAsync(&g.xscratch, cap, g.pool, g.xfer)) != cudaSuccess) return e;
         g.xscratch_cap = cap;
     }
-    const bool parts = a->part && a->part_end > 0 && a->part_end < a->n;
+    const bool parts = has_parts(a);
     if ((e = cudaStreamWaitEvent(g.xfer, parts ? a->part : a->ready, 0)) != cudaSuccess) return e;
     *buf = g.xscratch;
     *st = g.xfer;
@@ -251,22 +270,31 @@ View export_view(const_ft_ge25519_array a, size_t off = 0) { return View{a->plan
 // An export to host memory: conv(out, view, count, stream) writes bpp bytes
 // per point into the export buffer, which is copied to mem.  Where the call
 // that wrote a marked a first part, that part is converted and copied as
-// soon as it is written, then the rest after the mark.
+// soon as it is written, then the rest after the mark.  host_conv, where there
+// is one, writes pinned memory itself, beside its own arithmetic and with no
+// copy after it (folded points: 16 29 -> 26 us, 65,536 49 -> 39, 1,048,576 280
+// -> 219, of which the host link takes 174).  Its stores of 512 bytes a warp
+// are what makes that the faster way: of single 32-byte sectors 1,048,576
+// points take 485 us, and the raw conversion's 4-byte stores 13.1 ms against
+// 1.24 with the copy.  Not where a first part is marked: long ladders still run
+// then, and the copy leaves them the SMs (both halves of 524,288 ciphertexts
+// multiplied and exported 20.50 ms against 20.57).
 template <class Conv>
-ft_error export_to_host(uint8_t *mem, const_ft_ge25519_array a, size_t bpp, Conv conv)
+ft_error export_to_host(uint8_t *mem, const_ft_ge25519_array a, size_t bpp, Conv conv, Conv host_conv = nullptr)
 {
     const size_t n = a->n;
+    uint8_t *const direct = host_conv && !has_parts(a) ? device_view_of_host(mem, n * bpp) : nullptr;
     void *s;
     cudaStream_t st;
     size_t cut;
-    CK(export_begin(a, align256(n * bpp), &s, &st, &cut));
+    CK(export_begin(a, direct ? 0 : align256(n * bpp), &s, &st, &cut));
     size_t start = 0;
     for (const size_t end : {cut, n}) {
         if (end == start) continue;
         if (start) CK(cudaStreamWaitEvent(st, a->ready, 0));
-        uint8_t *buf = (uint8_t *)s + start * bpp;
-        CK(conv(buf, export_view(a, start), end - start, st));
-        CK(cudaMemcpyAsync(mem + start * bpp, buf, (end - start) * bpp, cudaMemcpyDeviceToHost, st));
+        uint8_t *buf = (direct ? direct : (uint8_t *)s) + start * bpp;
+        CK((direct ? host_conv : conv)(buf, export_view(a, start), end - start, st));
+        if (!direct) CK(cudaMemcpyAsync(mem + start * bpp, buf, (end - start) * bpp, cudaMemcpyDeviceToHost, st));
         start = end;
     }
     CK(cudaStreamSynchronize(st));
@@ -750,7 +778,7 @@ ft_error ft_array_to_bytes_folded(uint8_t *mem, size_t n_bytes, const_ft_ge25519
     size_t n = array->n;
     if (n_bytes / FT_FOLDED_POINT_BYTES < n) return FT_ERR_INSUFFICIENT_SPACE;
     if (n == 0) return FT_ERR_NO_ERROR;
-    return export_to_host(mem, array, 32, ft::encode);
+    return export_to_host(mem, array, 32, ft::encode, ft::encode_to_host);
 }
 
 ft_error ft_array_to_bytes_affine(uint8_t *mem, size_t n_bytes, const_ft_ge25519_array array)

@@ -115,6 +115,7 @@ cudaError_t gather_range(View dst, View src, size_t start, size_t step, size_t n
 cudaError_t scatter_range(View dst, View src, size_t start, size_t step, size_t n, cudaStream_t st);
 cudaError_t copy_points(View dst, View src, size_t n, cudaStream_t st);
 cudaError_t encode(uint8_t *d_out32, View v, size_t n, cudaStream_t st);
+cudaError_t encode_to_host(uint8_t *out32, View v, size_t n, cudaStream_t st); // out32: device_view_of_host's
 cudaError_t decode(View v, const uint8_t *d_in32, size_t n, long long *d_bad, cudaStream_t st);
 cudaError_t to_affine(uint8_t *d_out64, View v, size_t n, cudaStream_t st);
 cudaError_t from_affine(View v, const uint8_t *d_in64, size_t n, cudaStream_t st);

@@ -226,25 +226,37 @@ FT_DEV void use_z(fe &z, uint32_t &zero_mask, const uint4 w[2])
     fe_cmov(z, one, zero_mask);
 }
 
+// The lanes of a warp, converged, emit its points i, lane l the point l past a
+// multiple of 32, below n.
 struct EmitFolded {
-    static constexpr int WORDS = 2; // uint4 words per point
-    FT_DEV static void emit(uint4 *o, const fe &x, const fe &y)
+    // Lanes 16 apart trade half of their 32 bytes, so that a store instruction
+    // of the warp writes 512 contiguous bytes: the output may be host memory.
+    FT_DEV static void emit(uint4 *o, size_t i, size_t n, const fe &x, const fe &y)
     {
         fe yc;
         fe_canon(yc, y);
         yc.v[7] ^= fe_isnegative(x) << 31;
-        o[0] = u4_lo(yc);
-        o[1] = u4_hi(yc);
+        const uint4 a = u4_lo(yc), b = u4_hi(yc);
+        const unsigned up = threadIdx.x >> 4 & 1u;
+        uint4 t = up ? a : b;
+        t.x = __shfl_xor_sync(0xffffffffu, t.x, 16);
+        t.y = __shfl_xor_sync(0xffffffffu, t.y, 16);
+        t.z = __shfl_xor_sync(0xffffffffu, t.z, 16);
+        t.w = __shfl_xor_sync(0xffffffffu, t.w, 16);
+        const size_t e = i - 16 * up; // lane l < 16 and l + 16: the points e and e + 16
+        if (e < n) o[2 * e + up] = up ? t : a;
+        if (e + 16 < n) o[2 * (e + 16) + up] = up ? b : t;
     }
 };
 
 struct EmitAffine {
-    static constexpr int WORDS = 4;
-    FT_DEV static void emit(uint4 *o, const fe &x, const fe &y)
+    FT_DEV static void emit(uint4 *o, size_t i, size_t n, const fe &x, const fe &y)
     {
         fe xc, yc;
         fe_canon(xc, x);
         fe_canon(yc, y);
+        if (i >= n) return;
+        o += 4 * i;
         o[0] = u4_lo(xc);
         o[1] = u4_hi(xc);
         o[2] = u4_lo(yc);
@@ -310,10 +322,8 @@ __global__ void __launch_bounds__(ZINV_NT) k_zinv(uint4 *out, const uint4 *p, si
         fe zero;
         fe_0(zero);
         fe_cmov(zinv, zero, zm);
-        if (i < n) {
-            fe_mul_x2(x, x, zinv, y, y, zinv);
-            Emit::emit(out + Emit::WORDS * i, x, y);
-        }
+        fe_mul_x2(x, x, zinv, y, y, zinv);
+        Emit::emit(out, i, n, x, y);
     }
 }
 
@@ -629,22 +639,26 @@ cudaError_t validate(View v, size_t n, long long *bad, cudaStream_t st) { FT_LAU
 // Measured (n: this K, one point a thread, the earlier 8 points per chain of
 // 254 squarings): 16: 25, 25, 90 us; 65,536: 31 (K = 4), 71, 87 us;
 // 200,003: 47 (12), 177, 88 us; 1,048,576: 158 (12), 838, 314 us.
-static constexpr int ZINV_MAX_K = 18;
-static int zinv_points(size_t n)
+// Into host memory a launch takes at least what the host link does, and blocks
+// that start one after another keep it busy: threads of 6 points at most
+// (1,048,576 folded points, the call: 253 us at 18, 219 at 6, 217 at 4;
+// 4,194,304: 852, 755, 762).
+static constexpr int ZINV_MAX_K = 18, ZINV_HOST_K = 6;
+static int zinv_points(size_t n, int max_k)
 {
     const size_t per_sm = (size_t)sm_count() * ZINV_NT;
     for (size_t blocks = 1; blocks <= 3; ++blocks) {
         const size_t k = (n + blocks * per_sm - 1) / (blocks * per_sm);
-        if (k <= ZINV_MAX_K) return (int)k;
+        if (k <= (size_t)max_k) return (int)k;
     }
-    return ZINV_MAX_K;
+    return max_k;
 }
 
 template <class Emit>
-static cudaError_t zinv_launch(uint8_t *o, View v, size_t n, cudaStream_t st)
+static cudaError_t zinv_launch(uint8_t *o, View v, size_t n, cudaStream_t st, int max_k = ZINV_MAX_K)
 {
     if (n == 0) return cudaSuccess;
-    const int K = zinv_points(n);
+    const int K = zinv_points(n, max_k);
     const size_t smem = (size_t)(K - 1) * 2 * ZINV_NT * sizeof(uint4);
     const unsigned grid = (unsigned)((n + (size_t)ZINV_NT * K - 1) / ((size_t)ZINV_NT * K));
     static SmemAttr attr;
@@ -655,6 +669,10 @@ static cudaError_t zinv_launch(uint8_t *o, View v, size_t n, cudaStream_t st)
 }
 
 cudaError_t encode(uint8_t *o, View v, size_t n, cudaStream_t st) { return zinv_launch<EmitFolded>(o, v, n, st); }
+cudaError_t encode_to_host(uint8_t *o, View v, size_t n, cudaStream_t st)
+{
+    return zinv_launch<EmitFolded>(o, v, n, st, ZINV_HOST_K);
+}
 cudaError_t to_affine(uint8_t *o, View v, size_t n, cudaStream_t st) { return zinv_launch<EmitAffine>(o, v, n, st); }
 
 cudaError_t copy_points(View d, View s, size_t n, cudaStream_t st)

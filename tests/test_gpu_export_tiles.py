@@ -2,6 +2,8 @@
 32 points, blocks of 128, one to 18 points per inversion and one to three
 blocks per SM (the lengths are those of 152 SMs), with a zero Z in some of
 the products.  Exact: every byte against the oracle."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -28,3 +30,20 @@ def test_export_lengths(ft, pool, n):
     a = ft.Array.from_packed(pts).get_subset(idx)
     assert (a.to_bytes_folded() == enc[idx]).all()
     assert (a.to_bytes_affine() == aff[idx]).all()
+
+
+# where the encodings go: pinned memory on a 16-byte boundary is written by the
+# kernel itself, past a guard that it leaves alone; any other through a copy
+@pytest.mark.parametrize("pinned,shift", [(True, 0), (True, 16), (True, 8), (True, 1), (False, 0)])
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 4097, WAVE + 1])
+def test_export_destinations(ft, pool, n, pinned, shift):
+    torch = pytest.importorskip("torch")
+    pts, enc, _ = pool
+    idx = np.arange(n) % len(pts)
+    a = ft.Array.from_packed(pts).get_subset(idx)
+    buf = torch.full((32 * n + 64,), 0xA5, dtype=torch.uint8)
+    buf = buf.pin_memory() if pinned else buf
+    ft.check(ft.api.lib().ft_array_to_bytes_folded(ctypes.c_void_p(buf.data_ptr() + shift), 32 * n, a.handle))
+    out = buf.numpy()
+    assert (out[shift:shift + 32 * n].reshape(n, 32) == enc[idx]).all()
+    assert (out[:shift] == 0xA5).all() and (out[shift + 32 * n:] == 0xA5).all()
