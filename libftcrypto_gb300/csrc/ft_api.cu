@@ -141,9 +141,9 @@ bool host_is_pinned(const void *p)
     return at.type == cudaMemoryTypeHost;
 }
 
-// Where a kernel may write the caller's `bytes` bytes itself: pinned memory as
-// the device addresses it, 16-byte aligned; else nullptr.
-uint8_t *device_view_of_host(uint8_t *p, size_t bytes)
+// Where a kernel may read or write the caller's `bytes` bytes itself: pinned
+// memory as the device addresses it, 16-byte aligned; else nullptr.
+uint8_t *device_view_of_host(const uint8_t *p, size_t bytes)
 {
     cudaPointerAttributes at, end;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess ||
@@ -807,12 +807,16 @@ ft_error ft_array_from_bytes_folded(int64_t *res, ft_ge25519_array *array, const
     int64_t bad = -1;
     ft_error err = with_new_array(array, n, [&](ft_ge25519_array a) -> ft_error {
         if (n == 0) return FT_ERR_NO_ERROR;
-        void *s;
-        CK(scratch(&s, align256(n_bytes)));
-        CK(h2d(s, mem, n_bytes));
+        const uint8_t *in = device_view_of_host(mem, n_bytes);
+        if (!in) {
+            void *s;
+            CK(scratch(&s, align256(n_bytes)));
+            CK(h2d(s, mem, n_bytes));
+            in = (const uint8_t *)s;
+        }
         ft_error e2 = status_reset();
         if (e2) return e2;
-        CK(ft::decode(ft::view_of(a), (const uint8_t *)s, n, g.d_status, g.stream));
+        CK(ft::decode(ft::view_of(a), in, n, g.d_status, g.stream));
         return status_read(&bad);
     });
     if (err) return err;

@@ -327,6 +327,11 @@ __global__ void __launch_bounds__(ZINV_NT) k_zinv(uint4 *out, const uint4 *p, si
     }
 }
 
+// Bound by the chain of 254 squarings per point.  `in` may be the caller's
+// pinned memory: 32 bytes of a point across the host link wait behind the other
+// warps' squarings, where a copy before the launch and the wait for it cost the
+// call 28 us for 200,003 points (417 -> 389 us; 1,048,576: 1,969 -> 1,808; 16: 74
+// -> 65).  (The next point's 32 bytes loaded a point ahead: 396 us, spills.)
 __global__ void __launch_bounds__(128) k_decode(uint4 *p, size_t s, const uint4 *in, size_t n, long long *bad)
 {
     FT_GRID_LOOP(i, n)

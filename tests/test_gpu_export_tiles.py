@@ -47,3 +47,26 @@ def test_export_destinations(ft, pool, n, pinned, shift):
     out = buf.numpy()
     assert (out[shift:shift + 32 * n].reshape(n, 32) == enc[idx]).all()
     assert (out[:shift] == 0xA5).all() and (out[shift + 32 * n:] == 0xA5).all()
+
+
+# and where they come from: pinned memory on a 16-byte boundary is read by the
+# kernel itself, the rest through a copy; a warp's, a block's and a launch's
+# edges, and more points than a launch has threads
+@pytest.mark.parametrize("pinned,shift", [(True, 0), (True, 16), (True, 8), (False, 0)])
+@pytest.mark.parametrize("n", [1, 33, 129, 8 * WAVE + 1])
+def test_decode_sources(ft, pool, n, pinned, shift):
+    torch = pytest.importorskip("torch")
+    _, enc, _ = pool
+    idx = np.arange(n) % len(enc)
+    buf = torch.full((32 * n + 64,), 0xA5, dtype=torch.uint8)
+    buf = buf.pin_memory() if pinned else buf
+    buf.numpy()[shift:shift + 32 * n] = enc[idx].ravel()
+    arr, bad = ctypes.c_void_p(), ctypes.c_int64()
+    lib = ft.api.lib()
+    err = lib.ft_array_from_bytes_folded(ctypes.byref(bad), ctypes.byref(arr), ctypes.c_void_p(buf.data_ptr() + shift), 32 * n)
+    want, at = ft.Array.from_bytes_folded(enc[idx])
+    assert err == 0 and bad.value == at
+    out = np.zeros((n, 32), np.uint8)
+    ft.check(lib.ft_array_to_bytes_folded(out.ctypes.data_as(ctypes.c_void_p), out.size, arr))
+    lib.ft_array_free(arr)
+    assert (out == want.to_bytes_folded()).all()
