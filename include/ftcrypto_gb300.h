@@ -19,7 +19,10 @@ ft_error ftx_last_error(void);
 
 /* The CUDA runtime error (a cudaError_t value) behind the most recent
  * FT_ERR_INTERNAL_LIBRARY_ERROR or FT_ERR_OUT_OF_MEMORY, 0 if none; a
- * diagnostic only. */
+ * diagnostic only.  cudaErrorLaunchTimeout (702) also stands for a kernel of
+ * this library that gave up a wait with a limit: arrays written since may not
+ * hold points, and every later call, and every call that then waits for the
+ * GPU, returns FT_ERR_INTERNAL_LIBRARY_ERROR until the process ends. */
 int ftx_last_cuda_error(void);
 
 /* The library's CUDA stream (a cudaStream_t) on which every call runs. */

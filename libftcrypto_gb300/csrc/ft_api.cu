@@ -46,7 +46,8 @@ struct Ctx {
     uint64_t key_clock = 0;
     ft::CombTable b; // B's table (fixed-base products)
     // set by a kernel whose bounded wait ran out (mapped host memory): its
-    // results are not valid, and every later call reports it
+    // results are not valid.  Every later call reports it when it begins, and
+    // every call that waits for the GPU when it has waited (wait_for)
     volatile int *fault = nullptr;
     int *d_fault = nullptr;
     void *dlog_mem = nullptr;     // decryption table of j*B, j < dlog.m_max
@@ -91,13 +92,25 @@ ft_error map_err(cudaError_t e)
         if (_e != cudaSuccess) return map_err(_e);      \
     } while (0)
 
+// cudaErrorLaunchTimeout once a kernel of this library has given up a bounded
+// wait (Ctx::fault)
+cudaError_t gave_up() { return *g.fault ? cudaErrorLaunchTimeout : cudaSuccess; }
+
+// Waits for what is queued on st.  An error too if a kernel gave up: what the
+// caller was about to hand out may come from it.
+cudaError_t wait_for(cudaStream_t st)
+{
+    const cudaError_t e = cudaStreamSynchronize(st);
+    return e != cudaSuccess ? e : gave_up();
+}
+
 #define ENSURE_INIT()                                   \
     do {                                                \
         if (!g.inited) {                                \
             ft_error _ie = ft_crypto_init();            \
             if (_ie) return _ie;                        \
         }                                               \
-        if (*g.fault) return FT_ERR_INTERNAL_LIBRARY_ERROR; \
+        CK(gave_up());                                  \
     } while (0)
 
 cudaError_t dev_alloc(void **p, size_t bytes)
@@ -166,7 +179,7 @@ cudaError_t h2d(void *dst, const void *src, size_t bytes)
     if (e != cudaSuccess) return e;
     // a pageable source is staged before cudaMemcpyAsync returns; a pinned
     // one is read by DMA later, so wait for it
-    if (host_is_pinned(src)) e = cudaStreamSynchronize(g.stream);
+    if (host_is_pinned(src)) e = wait_for(g.stream);
     return e;
 }
 
@@ -177,7 +190,7 @@ cudaError_t d2h(void *dst, const void *src, size_t bytes, cudaStream_t st = null
         cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
         if (e != cudaSuccess) return e;
     }
-    return cudaStreamSynchronize(st);
+    return wait_for(st);
 }
 
 static cudaError_t record_on_stream(cudaEvent_t *ev, cudaStream_t st)
@@ -297,8 +310,8 @@ ft_error export_to_host(uint8_t *mem, const_ft_ge25519_array a, size_t bpp, Conv
         if (!direct) CK(cudaMemcpyAsync(mem + start * bpp, buf, (end - start) * bpp, cudaMemcpyDeviceToHost, st));
         start = end;
     }
-    CK(cudaStreamSynchronize(st));
-    return *g.fault ? FT_ERR_INTERNAL_LIBRARY_ERROR : FT_ERR_NO_ERROR;
+    CK(wait_for(st));
+    return FT_ERR_NO_ERROR;
 }
 
 // Copies `bytes` of pinned host memory into one of two staging buffers on
@@ -1206,7 +1219,7 @@ void *ftx_stream(void)
 ft_error ftx_synchronize(void)
 {
     ENSURE_INIT();
-    CK(cudaStreamSynchronize(g.stream));
+    CK(wait_for(g.stream));
     return FT_ERR_NO_ERROR;
 }
 
@@ -1307,7 +1320,7 @@ static ft_error encrypt_from_host(ft_ge25519_array a, ft_ge25519_array b, const 
         CK(cudaMemcpyAsync(&acc, dacc, sizeof acc, cudaMemcpyDeviceToHost, g.xfer));
     }
     // the caller may reuse its buffers: both parts are copied
-    CK(cudaStreamSynchronize(g.xfer));
+    CK(wait_for(g.xfer));
     return bits < 64 && (acc >> bits) ? FT_ERR_BAD_SIZE : FT_ERR_NO_ERROR;
 }
 
@@ -1556,7 +1569,7 @@ ft_error ftx_server_pk_table(const uint8_t *pk, CombTable *table)
     }
     ft_error err = build_key_table(*table, pk);
     if (!err) {
-        e = cudaStreamSynchronize(g.stream);
+        e = wait_for(g.stream);
         if (e != cudaSuccess) err = map_err(e);
     }
     if (err) {
@@ -1641,7 +1654,7 @@ ft_error batch_upload(ftx_batch b)
     if (!b->items.empty())
         CK(cudaMemcpyAsync(b->d_items, dev_items.data(), dev_items.size() * sizeof(ft::BatchItem),
                            cudaMemcpyHostToDevice, g.stream));
-    CK(cudaStreamSynchronize(g.stream));
+    CK(wait_for(g.stream));
     CK(ft::batch_prepare(b->w));
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(g.stream, cudaStreamCaptureModeThreadLocal));
