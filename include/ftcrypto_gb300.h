@@ -195,7 +195,7 @@ typedef struct {
     ft_ge25519_array c1, c2; /* RERAND, SMUL (updated); SEGSUM (source) */
 } ftx_request;
 typedef struct {
-    ft_error err;
+    ft_error err;            /* c1 and c2 of ENCRYPT and SEGSUM are NULL with an error */
     ft_ge25519_array c1, c2; /* the request's output arrays */
     double queue_ms;         /* submit -> admitted */
     double latency_ms;       /* submit -> GPU work complete */

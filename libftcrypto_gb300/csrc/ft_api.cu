@@ -1559,6 +1559,8 @@ const CombTable &base_table() { return g.b; }
 
 int *fault_word() { return g.d_fault; }
 
+bool kernel_gave_up() { return gave_up() != cudaSuccess; }
+
 // the table of a public key for a server (cudaMalloc'd; the server frees them)
 ft_error ftx_server_pk_table(const uint8_t *pk, CombTable *table)
 {

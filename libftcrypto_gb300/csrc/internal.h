@@ -138,6 +138,7 @@ struct CombTable {
 // B's table and the fault word of the library (ft_api.cu)
 const CombTable &base_table();
 int *fault_word();
+bool kernel_gave_up(); // the word is set
 cudaError_t comb_table(CombTable t, View q, cudaStream_t st); // of element 0 of q
 // (fault: a word that a kernel sets, and nothing clears, when a bounded wait
 // ran out and its results are not valid)

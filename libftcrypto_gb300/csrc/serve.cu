@@ -131,6 +131,7 @@ struct ftx_server_s {
     ft_error dispatch(Req *q, Slot &sl);
     Slot *free_slot(bool express);
     void admit(std::unique_lock<std::mutex> &lk, Req *q, Slot *sl);
+    void fail(Req *q, Slot *sl, ft_error err);
     void loop();
 };
 
@@ -286,7 +287,13 @@ void ftx_server_s::admit(std::unique_lock<std::mutex> &lk, Req *q, Slot *sl)
     ft_error err = dispatch(q, *sl);
     lk.lock();
     if (!err) return;
-    // finish q with the error; its memory is released in stream order
+    q->t_done = Clock::now();
+    fail(q, sl, err);
+}
+
+// finish q, on sl, with an error; its memory is released in stream order
+void ftx_server_s::fail(Req *q, Slot *sl, ft_error err)
+{
     q->res.err = err;
     if (q->r.op == FTX_REQ_ENCRYPT || q->r.op == FTX_REQ_SEGSUM) {
         for (ft_ge25519_array *a : {&q->res.c1, &q->res.c2})
@@ -301,7 +308,6 @@ void ftx_server_s::admit(std::unique_lock<std::mutex> &lk, Req *q, Slot *sl)
     in_use -= q->bytes + q->out_bytes;
     running--;
     sl->req = nullptr;
-    q->t_done = Clock::now();
     q->finished = true;
     cv_done.notify_all();
 }
@@ -315,6 +321,10 @@ void ftx_server_s::loop()
         for (Slot &sl : slots) {
             Req *q = sl.req;
             if (!q || !q->done) continue;
+            if (ft::kernel_gave_up()) { // one of its own or of those that wrote its inputs
+                fail(q, &sl, FT_ERR_INTERNAL_LIBRARY_ERROR);
+                continue;
+            }
             for (void *p : q->tmp) cudaFreeAsync(p, sl.st);
             q->tmp.clear();
             in_use -= q->bytes + q->out_bytes;

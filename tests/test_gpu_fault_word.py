@@ -91,3 +91,29 @@ def test_set_before_a_call(ft, have, word, name):
     with pytest.raises(ft.FtError) as e:
         {**ENTRY, **WAITING}[name](ft, have)
     assert e.value.code == INTERNAL
+
+
+def test_server_request(ft, have, word):
+    """A request that runs when a kernel gives up ends with the error: its new
+    arrays are nobody's, its bytes are back in the budget."""
+    g, n = have["g"], 5000
+    m, r = synth.plaintexts(g, n, 1), synth.scalars_mod_L(g, n)
+    srv = ft.Server(have["pk"], 1 << 30, slots=2)
+    c1, c2, _, _ = srv.wait(srv.submit_encrypt(m, r, 1))
+    held = srv.stats()[0]
+    off = synth.csr_offsets(g, n, 100)
+    for submit in (lambda: srv.submit_encrypt(m, r, 1), lambda: srv.submit_rerand(c1, c2, r),
+                   lambda: srv.submit_smul(c1, c2, r), lambda: srv.submit_segsum(c1, c2, off)):
+        for _ in range(8):  # 40 ms of work that the request waits for
+            have["long"].scale(have["sk"])
+        ticket = submit()
+        word.value = 1
+        with pytest.raises(ft.FtError) as e:
+            srv.wait(ticket)
+        assert e.value.code == INTERNAL and srv.stats() == (held, 0, 0)
+        word.value = 0
+    d1, d2, _, _ = srv.wait(srv.submit_encrypt(m, r, 1))
+    assert srv.stats()[0] == 2 * held
+    srv.release(c1, c2, d1, d2)
+    assert srv.stats() == (0, 0, 0)
+    srv.close()
