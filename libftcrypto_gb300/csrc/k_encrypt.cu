@@ -25,6 +25,7 @@
 #include "points.cuh"
 #include "enc_comb.cuh"
 #include "comb256.cuh"
+#include "comb_roles.cuh"
 #include "fe_inv.cuh"
 #include "quad.cuh"
 #include "umma.cuh"
@@ -186,7 +187,7 @@ struct CombSmem {
     static constexpr int NT = 128 * G;
     static constexpr uint32_t A = COMB_N, PER_WG = COMB_N + COMB_K / 2 + 8, COLS = G == 1 ? 256 : 512;
     static_assert(G * PER_WG <= COLS, "tensor memory");
-    static constexpr size_t B = 0, MAGIC = 3 * (size_t)COMB_ROW_BYTES,
+    static constexpr size_t B = 0, MAGIC = COMB_BUFS * (size_t)COMB_ROW_BYTES,
                             DIG = MAGIC + 2 * COMB_CHUNK, X = DIG + (size_t)8 * NT * 4;
     static constexpr size_t USED = X + (G == 1 ? 2 * (size_t)8 * NT * 16 : 0); // X: points from the cluster's others
     static constexpr size_t BYTES = std::max(USED, (size_t)(G == 1 ? 80 : 116) * 1024);
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(128 * (G + 1), SPLIT ? 2 : 1) k_comb256(CombJo
 {
     using S = CombSmem<G>;
     extern __shared__ __align__(128) uint8_t sm[];
-    __shared__ uint64_t full[3], empty[3], done[G], ready[G];
+    __shared__ uint64_t full[COMB_BUFS], empty[COMB_BUFS], done[G], ready[G];
     __shared__ uint32_t s_taddr;
     const int tid = threadIdx.x, wg = tid >> 7, warp = tid >> 5;
     const int nr = j.sc ? COMB_ROWS : 0;
@@ -235,7 +236,7 @@ __global__ void __launch_bounds__(128 * (G + 1), SPLIT ? 2 : 1) k_comb256(CombJo
     if (warp == 0) tmem_alloc(&s_taddr, S::COLS);
     if (tid == 0) {
 #pragma unroll
-        for (int b = 0; b < 3; ++b) {
+        for (int b = 0; b < (int)COMB_BUFS; ++b) {
             mbar_init(&full[b], 1);
             mbar_init(&empty[b], G);
         }
@@ -257,42 +258,9 @@ __global__ void __launch_bounds__(128 * (G + 1), SPLIT ? 2 : 1) k_comb256(CombJo
     if (SPLIT) cluster_sync(); // every block of it runs
 
     ge_p3 h;
-    if (wg == G && warp - 4 * G == 3) { // the loads
-        if ((tid & 31) == 0) {
-            unsigned loads = 0, buf = 0, use = 0;
-            bool bad = false;
-#pragma unroll 1
-            for (unsigned tile = tile0; tile < tiles && !bad; tile += hop) {
-                const int h = j.h1 - 1 - (int)(tile / per_half);
-                int r0, r1;
-                span(h, r0, r1);
-#pragma unroll 1
-                for (int t = r0; t < r1; ++t, ++loads) {
-                    const uint8_t *src = t < nr ? CombJob::pick(j.tr, h) + (size_t)(nr - 1 - t) * COMB_ROW_BYTES
-                                                : j.tm + (size_t)(t - nr) * COMB_ROW_BYTES;
-                    // the buffer's use before this one
-                    if (use && !mbar_wait<COMB_SLEEP>(&empty[buf], (use - 1) & 1)) {
-                        bad = true;
-                        break;
-                    }
-                    mbar_expect(&full[buf], COMB_ROW_BYTES);
-                    bulk_load(sm + S::B + buf * COMB_ROW_BYTES, src, COMB_ROW_BYTES, &full[buf]);
-                    if (++buf == 3) {
-                        buf = 0;
-                        ++use;
-                    }
-                }
-            }
-            // the last copies have landed before the block ends
-#pragma unroll 1
-            for (unsigned k = loads < 3 ? 0 : loads - 3; k < loads; ++k)
-                if (!mbar_wait<COMB_SLEEP>(&full[k % 3], (k / 3) & 1)) bad = true;
-            if (bad) *(volatile int *)fault = 1;
-        }
-        __syncwarp();
-    } else if (wg == G) { // the products of warpgroup g
-        const int g = warp - 4 * G;
-        if (g < G && (tid & 31) == 0) {
+    if (wg == G) { // one thread each: warp 3 the loads, warp g the products of warpgroup g
+        const int role = warp - 4 * G;
+        if ((tid & 31) == 0 && (role < G || role == 3)) {
             unsigned steps = 0;
 #pragma unroll 1
             for (unsigned tile = tile0; tile < tiles; tile += hop) {
@@ -300,28 +268,45 @@ __global__ void __launch_bounds__(128 * (G + 1), SPLIT ? 2 : 1) k_comb256(CombJo
                 span(j.h1 - 1 - (int)(tile / per_half), r0, r1);
                 steps += r1 - r0;
             }
-            const uint32_t dt = s_taddr + S::PER_WG * g;
-            unsigned buf = 0, use = 0; // the step's buffer, and that buffer's use
-#pragma unroll 1
-            for (unsigned q = 0; q < steps; ++q) {
-                if (!mbar_wait<COMB_SLEEP>(&full[buf], use & 1) || !mbar_wait<COMB_SLEEP>(&ready[g], q & 1)) {
-                    *(volatile int *)fault = 1;
-                    break;
-                }
-                tmem_fence_after();
-                const uint64_t bd = umma_desc(smem_addr(sm + S::B + buf * COMB_ROW_BYTES), COMB_CHUNK, 128);
-                umma_f16_ta(dt, dt + S::A + COMB_K / 2, umma_desc(smem_addr(sm + S::MAGIC), COMB_CHUNK, 128), COMB_IDESC,
-                            false);
+            auto wait_full = [&](unsigned b, unsigned parity) { return mbar_wait<COMB_SLEEP>(&full[b], parity); };
+            bool ok;
+            if (role == 3) {
+                unsigned tile = tile0;
+                int half = j.h1 - 1 - (int)(tile / per_half), t, end;
+                span(half, t, end);
+                ok = comb_load(
+                    steps, wait_full,
+                    [&](unsigned b, unsigned parity) { return mbar_wait<COMB_SLEEP>(&empty[b], parity); },
+                    [&](unsigned b) {
+                        if (t == end) {
+                            tile += hop;
+                            half = j.h1 - 1 - (int)(tile / per_half);
+                            span(half, t, end);
+                        }
+                        const uint8_t *src = t < nr ? CombJob::pick(j.tr, half) + (size_t)(nr - 1 - t) * COMB_ROW_BYTES
+                                                    : j.tm + (size_t)(t - nr) * COMB_ROW_BYTES;
+                        ++t;
+                        mbar_expect(&full[b], COMB_ROW_BYTES);
+                        bulk_load(sm + S::B + b * COMB_ROW_BYTES, src, COMB_ROW_BYTES, &full[b]);
+                    });
+            } else {
+                const uint32_t dt = s_taddr + S::PER_WG * role;
+                ok = comb_issue(
+                    steps, wait_full, [&](unsigned parity) { return mbar_wait<COMB_SLEEP>(&ready[role], parity); },
+                    [&](unsigned parity) { return mbar_wait<COMB_SLEEP>(&done[role], parity); },
+                    [&](unsigned b) {
+                        tmem_fence_after();
+                        const uint64_t bd = umma_desc(smem_addr(sm + S::B + b * COMB_ROW_BYTES), COMB_CHUNK, 128);
+                        umma_f16_ta(dt, dt + S::A + COMB_K / 2, umma_desc(smem_addr(sm + S::MAGIC), COMB_CHUNK, 128),
+                                    COMB_IDESC, false);
 #pragma unroll
-                for (int k = 0; k < COMB_K / 16; ++k)
-                    umma_f16_ta(dt, dt + S::A + 8u * k, bd + k * (2 * COMB_CHUNK >> 4), COMB_IDESC, true);
-                umma_commit(&done[g]);
-                umma_commit(&empty[buf]);
-                if (++buf == 3) {
-                    buf = 0;
-                    ++use;
-                }
+                        for (int k = 0; k < COMB_K / 16; ++k)
+                            umma_f16_ta(dt, dt + S::A + 8u * k, bd + k * (2 * COMB_CHUNK >> 4), COMB_IDESC, true);
+                        umma_commit(&done[role]);
+                        umma_commit(&empty[b]);
+                    });
             }
+            if (!ok) *(volatile int *)fault = 1;
         }
         __syncwarp();
     } else {

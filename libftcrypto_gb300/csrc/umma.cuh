@@ -9,7 +9,8 @@
 //
 // Every wait is bounded: mbar_wait gives up after a fixed number of polls and
 // says so, and the kernel then leaves its loops, waits (bounded again) for
-// its own copies and frees its tensor memory.
+// the copies and the products that it has started and frees its tensor memory
+// (comb_roles.cuh).
 #pragma once
 #include "tmem.cuh"
 
