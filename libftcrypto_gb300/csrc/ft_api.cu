@@ -16,6 +16,9 @@
 #include <set>
 #include <vector>
 
+#include <cuda.h>
+
+#include "host_view.h"
 #include "internal.h"
 #include "../../include/ftcrypto.h"
 #include "../../include/ftcrypto_gb300.h"
@@ -154,22 +157,38 @@ bool host_is_pinned(const void *p)
     return at.type == cudaMemoryTypeHost;
 }
 
-// Where a kernel may read or write the caller's `bytes` bytes itself: pinned
-// memory as the device addresses it, 16-byte aligned; else nullptr.
-uint8_t *device_view_of_host(const uint8_t *p, size_t bytes)
+// the block of pinned memory that holds p.  The runtime tells where the device
+// addresses p, only the driver how far the block goes; where the device's
+// addresses are others than the host's its range would be too: no answer.
+bool host_block(ft::HostBlock &b, const uint8_t *p)
 {
-    cudaPointerAttributes at, end;
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess ||
-        cudaPointerGetAttributes(&end, p + bytes - 1) != cudaSuccess) {
+    using GetAttributes = CUresult(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+    static GetAttributes *const get = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const cudaError_t e = cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &q);
+        if (e != cudaSuccess) cudaGetLastError();
+        return e == cudaSuccess && q == cudaDriverEntryPointSuccess ? (GetAttributes *)f : nullptr;
+    }();
+    cudaPointerAttributes at;
+    if (!get || cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         cudaGetLastError();
-        return nullptr;
+        return false;
     }
-    uint8_t *d = (uint8_t *)at.devicePointer;
-    if (at.type != cudaMemoryTypeHost || end.type != cudaMemoryTypeHost || !d || (uintptr_t)d % 16 ||
-        (uint8_t *)end.devicePointer != d + bytes - 1)
-        return nullptr;
-    return d;
+    if (at.type != cudaMemoryTypeHost || at.devicePointer != (const void *)p) return false;
+    CUdeviceptr start = 0;
+    size_t bytes = 0;
+    CUpointer_attribute what[2] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *to[2] = {&start, &bytes};
+    if (get(2, what, to, (CUdeviceptr)p) != CUDA_SUCCESS || !start) return false;
+    b.start = (const uint8_t *)start;
+    b.bytes = bytes;
+    b.device = (uint8_t *)at.devicePointer;
+    return true;
 }
+
+// where a kernel may read or write the caller's `bytes` bytes itself; else nullptr
+uint8_t *device_view_of_host(const uint8_t *p, size_t bytes) { return ft::device_view(p, bytes, host_block); }
 
 // copy from caller memory: the caller may reuse `src` when this returns
 cudaError_t h2d(void *dst, const void *src, size_t bytes)
