@@ -1,7 +1,7 @@
 // enc_comb.cuh — enc_ref_scalar, the scalar every fixed-base product uses, and
-// the fixed-base comb in signed radix 32 with a masked select, which the
-// kernels' comb in radix 256 (comb256.cuh) took the place of: the host tests
-// still check digits, table entries and products by it.
+// a fixed-base comb in signed radix 32 with a masked select.  No kernel runs
+// that comb (theirs is in radix 256, comb256.cuh): it is what the host tests
+// check the formulas and enc_ref_scalar by.
 //
 // A scalar a < 2^256 is written as ENC_ROWS = 52 digits d_i in [-16, 16):
 // b = a + sum_{i<52} 16 * 32^i (below 2^260), d_i = bits [5i, 5i+5) of b
@@ -59,19 +59,6 @@ FT_DEV void shr5_288(uint32_t c[9])
 
 // t = the entry |d| of a table row (ENC_ENTRIES entries), negated for d < 0;
 // the identity for d = 0; every entry is read and merged under its mask.
-// Eight entries per iteration of a rolled loop.  With the field arithmetic
-// of the time: 12.03 ms for the encryption of 1,048,576 plaintexts with
-// four, 12.06 with two, 12.33 with eight, 12.71 fully unrolled and 13.96
-// with one (instruction fetch and load latency); after the encryption
-// stopped keeping the digits of r and m in registers: 9.78 ms with four,
-// 9.90 with two, 9.72 with eight or sixteen.  Moving some entries to the multiply-add
-// pipe (products by 0/1 indicators) measured 1-3% slower at every grouping.
-#ifndef FT_ENC_SEL_GROUP
-#define FT_ENC_SEL_GROUP 8
-#endif
-static constexpr int ENC_SEL_GROUP = FT_ENC_SEL_GROUP;
-static_assert(ENC_ENTRIES % ENC_SEL_GROUP == 0, "select grouping");
-
 FT_DEV void enc_select(ge_precomp &t, int d, const uint4 *row)
 {
     const uint32_t bneg = (uint32_t)d >> 31;
@@ -82,22 +69,17 @@ FT_DEV void enc_select(ge_precomp &t, int d, const uint4 *row)
     const uint32_t id = babs == 0u ? 1u : 0u; // the identity (1, 1, 0)
     t.yplusx.v[0] = id;
     t.yminusx.v[0] = id;
-#pragma unroll 1
-    for (int k = 0; k < ENC_ENTRIES; k += ENC_SEL_GROUP) {
-#pragma unroll
-        for (int q = 0; q < ENC_SEL_GROUP; ++q) {
-            const uint4 *e = row + 6 * (k + q);
-            fe e0, e1, e2;
-            fe_from_u4(e0, e[0], e[1]);
-            fe_from_u4(e1, e[2], e[3]);
-            fe_from_u4(e2, e[4], e[5]);
-            const uint32_t m = ct_eq_mask(babs, (uint32_t)(k + q + 1));
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                t.yplusx.v[i] |= e0.v[i] & m;
-                t.yminusx.v[i] |= e1.v[i] & m;
-                t.xy2d.v[i] |= e2.v[i] & m;
-            }
+    for (int k = 0; k < ENC_ENTRIES; ++k) {
+        const uint4 *e = row + 6 * k;
+        fe e0, e1, e2;
+        fe_from_u4(e0, e[0], e[1]);
+        fe_from_u4(e1, e[2], e[3]);
+        fe_from_u4(e2, e[4], e[5]);
+        const uint32_t m = ct_eq_mask(babs, (uint32_t)(k + 1));
+        for (int i = 0; i < 8; ++i) {
+            t.yplusx.v[i] |= e0.v[i] & m;
+            t.yminusx.v[i] |= e1.v[i] & m;
+            t.xy2d.v[i] |= e2.v[i] & m;
         }
     }
     const uint32_t nm = 0u - bneg;

@@ -468,7 +468,8 @@ FT_DEV void fe_sqn(fe &h, const fe &f, int n)
     for (int i = 1; i < n; ++i) fe_sq(h, h);
 }
 
-// z^(p-2), the addition chain of fe25519_invert (sodium_fe.cu:1352-1408)
+// z^(p-2), the addition chain of fe25519_invert (sodium_fe.cu:1352-1408): what
+// the host tests compare with; kernels invert by division steps (fe_inv.cuh)
 FT_DEV void fe_invert(fe &out, const fe &z)
 {
     fe t0, t1, t2, t3;

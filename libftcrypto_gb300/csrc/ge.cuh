@@ -303,8 +303,8 @@ FT_DEV uint32_t ct_eq_mask(uint32_t a, uint32_t b)
     return 0u - ((x - 1u) >> 31); // all ones iff a == b (a, b < 2^31)
 }
 
-// (the selections that use it: ge_add_select in smul.cuh, enc_select in
-// enc_comb.cuh, each reading every entry and merging under masks, with no
+// (the selections that use it: ge_add_select in smul.cuh, k_smul_quad's in
+// k_smul.cu, each reading every entry and merging under masks, with no
 // address or branch depending on the digit)
 
 // ---- signed radix-16 digits (the recoding of sodium_ge.cu:693-708)

@@ -212,7 +212,7 @@ struct CombSmem {
 // 5.22 with comb_add.  (What is added to the multiplications is not hidden by
 // them: about a cycle an instruction.  The one-hot rows written by the issuing
 // warps instead: 5.69 against 5.45.)
-// SPLIT (G = 1): the blocks of a cluster (1, 2, 4 or 8) take a part of a tile's
+// SPLIT (G = 1): the blocks of a cluster (2, 4 or 8) take a part of a tile's
 // rows each, then add their points up in pairs, through the shared memory of
 // the lower block of each pair.
 template <int G, bool ACC, bool SPLIT>
@@ -472,7 +472,7 @@ static cudaError_t comb_launch(CombJob j, const CombTable *tr0, const CombTable 
     // two per SM at most.
     const size_t t = tiles(1);
     if (t <= sm) {
-        const unsigned parts = 8 * t <= 2 * sm ? 8 : 4 * t <= 2 * sm ? 4 : 2 * t <= 2 * sm ? 2 : 1;
+        const unsigned parts = 8 * t <= 2 * sm ? 8 : 4 * t <= 2 * sm ? 4 : 2;
         return launch_256<1, ACC, true>(j, t, parts, fault, st);
     }
     // Beyond, a round of a tile of 256 units per SM takes about 103 us, of 384

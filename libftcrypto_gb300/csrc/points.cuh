@@ -38,17 +38,6 @@ FT_DEV void st_p3(uint4 *__restrict__ p, size_t s, size_t i, const ge_p3 &r)
 }
 
 // warp shuffle of a whole point
-FT_DEV void shfl_down_p3(ge_p3 &o, const ge_p3 &v, int delta)
-{
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        o.X.v[k] = __shfl_down_sync(0xffffffffu, v.X.v[k], delta);
-        o.Y.v[k] = __shfl_down_sync(0xffffffffu, v.Y.v[k], delta);
-        o.Z.v[k] = __shfl_down_sync(0xffffffffu, v.Z.v[k], delta);
-        o.T.v[k] = __shfl_down_sync(0xffffffffu, v.T.v[k], delta);
-    }
-}
-
 FT_DEV void shfl_up_p3(ge_p3 &o, const ge_p3 &v, int delta)
 {
 #pragma unroll
@@ -57,17 +46,6 @@ FT_DEV void shfl_up_p3(ge_p3 &o, const ge_p3 &v, int delta)
         o.Y.v[k] = __shfl_up_sync(0xffffffffu, v.Y.v[k], delta);
         o.Z.v[k] = __shfl_up_sync(0xffffffffu, v.Z.v[k], delta);
         o.T.v[k] = __shfl_up_sync(0xffffffffu, v.T.v[k], delta);
-    }
-}
-
-FT_DEV void shfl_idx_p3(ge_p3 &o, const ge_p3 &v, int lane)
-{
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        o.X.v[k] = __shfl_sync(0xffffffffu, v.X.v[k], lane);
-        o.Y.v[k] = __shfl_sync(0xffffffffu, v.Y.v[k], lane);
-        o.Z.v[k] = __shfl_sync(0xffffffffu, v.Z.v[k], lane);
-        o.T.v[k] = __shfl_sync(0xffffffffu, v.T.v[k], lane);
     }
 }
 

@@ -7,7 +7,7 @@
 //       wherever the caller's accessor puts it (shared memory in the kernels).
 //   smul_ladder_u32 : the same ladder for scalars under a public bound, in
 //       fewer (and optionally narrower) windows.
-// The fixed-base comb is in enc_comb.cuh.
+// The fixed-base comb is in comb256.cuh.
 #pragma once
 #include "ge.cuh"
 #include "windows.h"

@@ -26,7 +26,7 @@ static_assert(u32_ladder_windows(32) == 9 && u32_ladder_windows(10) == 3 && u32_
                   u32_ladder_windows(10, 3) == 4 && u32_ladder_windows(10, 2) == 6,
               "window counts");
 
-// The radix-32 fixed-base comb (enc_comb.cuh): ENC_ROWS rows of ENC_ENTRIES
+// The radix-32 fixed-base comb of the host tests (enc_comb.cuh): ENC_ROWS rows of ENC_ENTRIES
 // entries (j+1) * 32^row * Q, and the rows a scalar below 2^bits needs
 // (bits <= 256): the smallest d with a + sum_{i<d} 16 * 32^i < 32^d for every
 // a < 2^bits, i.e. 15 * 32^d + 16 >= 31 * 2^bits.
