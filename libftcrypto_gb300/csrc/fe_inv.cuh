@@ -1,6 +1,14 @@
-// fe_inv.cuh — inversion mod p = 2^255 - 19 by division steps (Bernstein and
-// Yang, "Fast constant-time gcd computation and modular inversion", 2019, in
-// the variant that starts at delta = 1/2), constant time.
+// fe_inv.cuh — inversion mod p = 2^255 - 19 by division steps, constant time.
+//
+// The division steps, the transition matrices of several of them and their
+// use on d and e are Bernstein and Yang's ("Fast constant-time gcd computation
+// and modular inversion", 2019).  The variant that starts at delta = 1/2 and
+// its bound of 590 steps for 256 bits are P. Wuille's (safegcd-bounds, 2021).
+// The layout, nine signed limbs of 30 bits, 20 rounds of 30 steps, d and e kept
+// in (-2p, p) and brought into [0, p) in two additions at the end, is the one
+// that P. Dettman and P. Wuille describe for libsecp256k1 ("The safegcd
+// implementation in libsecp256k1 explained", 2021).  The steps by multiply-adds
+// and the split over the four lanes of a quad (quad_inv) are this library's.
 //
 // z^(p-2) is a chain of 254 squarings that nothing in one thread overlaps:
 // 75 us on a warp alone, whatever the number of points it serves; this takes

@@ -636,14 +636,16 @@ cudaError_t to_packed(uint8_t *o, View v, size_t n, cudaStream_t st) { FT_LAUNCH
 cudaError_t from_packed(View v, const uint8_t *in, size_t n, cudaStream_t st) { FT_LAUNCH(k_from_packed, n, 256, v.p, v.s, (const uint4 *)in, n); }
 cudaError_t validate(View v, size_t n, long long *bad, cudaStream_t st) { FT_LAUNCH(k_validate, n, 128, v.p, v.s, n, bad); }
 
-// Points per inversion: an inversion costs a warp scheduler 30,000 to 39,000
-// cycles (19 us alone) and a point in the loops about 5,000 (2 us), so the
-// points go one to a thread until every scheduler has a warp (sm_count x 128
-// threads), and then into longer threads: one block per SM up to 18 points
-// a thread, two, three (72 KB of shared memory each), each launch one wave.
-// Measured (n: this K, one point a thread, the earlier 8 points per chain of
-// 254 squarings): 16: 25, 25, 90 us; 65,536: 31 (K = 4), 71, 87 us;
-// 200,003: 47 (12), 177, 88 us; 1,048,576: 158 (12), 838, 314 us.
+// Points per inversion: a warp's inversions cost its scheduler 24,000 cycles
+// (12 us alone) and a point in the loops 1.5 us, so the points go one to a
+// thread until every scheduler has a warp (sm_count x 128 threads), and then
+// into longer threads: one block per SM up to 18 points a thread, two, three
+// (72 KB of shared memory each), each launch one wave.  Measured (n: this K; one
+// point a thread; 8; the earlier kernel's 8 points per chain of 254 squarings),
+// us a launch into device memory: 16: 15 (K = 1); 15; 26; 90.  65,536: 23 (4);
+// 44; 31; 87.  200,003: 38 (11); 112; 44; 88.  400,000: 51 (11); 209; 59.
+// 1,048,576: 96 (18); 529; 122; 314.  (No K from 1 to 18 was better than the
+// rule's by 1 us at eight lengths.)
 // Into host memory a launch takes at least what the host link does, and blocks
 // that start one after another keep it busy: threads of 6 points at most
 // (1,048,576 folded points, the call: 253 us at 18, 219 at 6, 217 at 4;

@@ -10,9 +10,11 @@
 //   * warp 0 allocates with tmem_alloc (whole warp), the address is published
 //     through shared memory behind tmem_sync_threads(), and warp 0 frees the
 //     same columns after a final tmem_sync_threads();
-//   * a kernel allocates only when it is the only CTA its SM can hold (its
-//     shared memory exceeds half of the SM's), so an allocation never waits
-//     for another CTA's columns;
+//   * the blocks of one kernel that its shared memory lets an SM hold take no
+//     more than its 512 columns together (all of them by the only block, or 256
+//     by each of two), so an allocation waits for no block of the same kernel;
+//     one of another kernel in another stream frees its columns when it ends
+//     and waits for no block that is not running, so the wait ends;
 //   * the .sync.aligned forms are executed by every thread of a warp
 //     together: the kernels run no divergent code around them;
 //   * loads complete inside the same asm statement (tcgen05.wait::ld), so the
